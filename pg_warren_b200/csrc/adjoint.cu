@@ -20,6 +20,7 @@
 #include "pagerank.h"
 #include "pull32.cuh"
 #include "pull_multi.cuh"
+#include "upload.h"
 
 namespace wc {
 
@@ -318,12 +319,19 @@ wc_status wc_pagerank_adjoint(wc_version* v, const wc_call* call, const wc_pager
   PageRankRun fwd;
   WC_TRY(fwd.setup(ctx, o, nullptr, nullptr));
   WC_TRY(fwd.run(ctx));
-  WC_TRY(ctx.finish());
+  WC_TRY(locality_status(ctx, ctx.finish()));
   uint32_t its = 0;
   WC_CUDA(cudaMemcpy(&its, fwd.s.iterations, 4, cudaMemcpyDeviceToHost), ctx.detail);
   if (o->max_iter == 0) its = 0;
-  const double* x = fwd.s.x[its & 1];
-  if (ranks_out) WC_CUDA(cudaMemcpy(ranks_out, x, n * 8, cudaMemcpyDefault), ctx.detail);
+  // The ranks and the out-weights by dense id, as the forward CSR numbers
+  // its rows, through buffers the solve is done with.
+  double *x = fwd.s.x[(its & 1) ^ 1], *out = fwd.s.msg[0];
+  WC_TRY(from_locality(v, ctx.stream, fwd.s.x[its & 1], x));
+  WC_TRY(from_locality(v, ctx.stream, fwd.s.out, out));
+  if (ranks_out) {
+    WC_CUDA(cudaMemcpyAsync(ranks_out, x, n * 8, cudaMemcpyDefault, ctx.stream), ctx.detail);
+    WC_CUDA(cudaStreamSynchronize(ctx.stream), ctx.detail);
+  }
   if (losses == 0) {
     if (iterations_out) iterations_out[0] = its;
     return WC_OK;
@@ -352,7 +360,7 @@ wc_status wc_pagerank_adjoint(wc_version* v, const wc_call* call, const wc_pager
   s.lam[1] = s.lam[0] + n * P;
   s.S = Sb->as<double>();
   s.C = Cb->as<double>();
-  s.out = fwd.s.out;
+  s.out = out;
   s.x = x;
   s.damping = o->damping;
   s.p = fwd.s.start;

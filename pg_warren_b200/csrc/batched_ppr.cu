@@ -550,7 +550,8 @@ wc_status tune_ppr(Ctx& ctx, uint32_t width, wc_schedule* best) {
   WC_CUDA(cudaMemcpyAsync(F->ptr, offs.data(), (sample + 1) * 8, cudaMemcpyHostToDevice, ctx.stream), ctx.detail);
   wc_pagerank_opts o{0.85, 1e-10, 1, -1, 10, nullptr};
   PageRankRun base;
-  WC_TRY(base.setup(ctx, &o, nullptr, nullptr, true));
+  WC_TRY(base.setup(ctx, &o, nullptr, nullptr));
+  WC_TRY(base.out_now(ctx));
   cudaEvent_t a, b;
   WC_CUDA(cudaEventCreate(&a), ctx.detail);
   WC_CUDA(cudaEventCreate(&b), ctx.detail);
@@ -601,7 +602,8 @@ wc_status wc_ppr_batched(wc_version* v, const wc_call* call, const wc_pagerank_o
     WC_CUDA(cudaMemcpy(nodes.data(), seed_nodes, nodes.size() * 8, cudaMemcpyDefault), ctx.detail);
   WC_TRY(ctx.begin());
   PageRankRun base;
-  WC_TRY(base.setup(ctx, o, nullptr, nullptr, true));
+  WC_TRY(base.setup(ctx, o, nullptr, nullptr));
+  WC_TRY(base.out_now(ctx));
   // Each set's personalisation (pagerank/mod.rs:155-199 with a seed of 1
   // on the set): the set's size summed in the reference's order is exact
   // (integers), then 1 / size, then 1 × that share.

@@ -1,16 +1,16 @@
-// locality.cu — a version's reverse CSR in locality order, for the pull
-// solvers whose cost is the gather of x over the entries (PageRank).
+// locality.cu — a version's reverse CSR in row order, for the solvers that
+// keep their per-node vectors in an order of their own (PageRank, the batched
+// personalised PageRank).
 //
-// The nodes are renumbered by out-degree, largest first (equal degrees in
-// dense-id order).  A pull over the reverse CSR reads x_j once per out-edge
-// of j, so the nodes gathered most often get the lowest numbers: their
-// values share 32-byte sectors and cache lines, and the most gathered of
-// them stay in each SM's L1.  Row k of the renumbered CSC is the reverse row
-// of node order[k] with its entries in their stored order and each source
-// renumbered perm[source]; a row's fold adds the same products in the same
-// order as over the plain CSC, so each row's result is the same bit for
-// bit.  A solver keeps its per-node vectors in the new numbering and
-// renumbers only at the boundary: inputs scattered in, results gathered out.
+// The nodes are renumbered by the length of their reverse rows, longest first
+// (equal lengths in dense-id order): the order in which the lane-major copy
+// (lanes.cu) deals rows to lanes, so a slice's 32 rows are 32 consecutive
+// values of every vector its epilogue reads and writes.  Row k of the
+// renumbered CSC is the reverse row of node order[k] with its entries in
+// their stored order and each source renumbered perm[source]; a row's fold
+// adds the same products in the same order as over the plain CSC, so each
+// row's result is the same bit for bit.  A solver renumbers only at the
+// boundary: inputs scattered in, results gathered out.
 // (The reference's own locality orders, graph/node_order/, renumber the
 // stored graph; this one is internal to the device copy.)
 #include <algorithm>
@@ -24,10 +24,10 @@
 
 namespace wc {
 
-__global__ void degree_keys_kernel(const uint32_t* fwd_off, uint32_t n, uint32_t* keys,
+__global__ void degree_keys_kernel(const uint32_t* off, uint32_t n, uint32_t* keys,
                                    uint32_t* ids) {
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    keys[i] = ~(fwd_off[i + 1] - fwd_off[i]);  // ascending keys: largest degree first
+    keys[i] = ~(off[i + 1] - off[i]);  // ascending keys: longest row first
     ids[i] = i;
   }
 }
@@ -61,6 +61,21 @@ __global__ void loc_entries_kernel(const uint32_t* order, const uint32_t* perm,
   }
 }
 
+// The lane-major copy's targets and hot nodes in the new numbers (a hot
+// target's slot stays).
+__global__ void loc_lanes_kernel(const uint32_t* targets, uint64_t places, const uint32_t* hot,
+                                 uint32_t hot_count, const uint32_t* perm, uint32_t* new_targets,
+                                 uint32_t* new_hot) {
+  const uint64_t first = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  const uint32_t hot_bit = hot_count ? kHotTarget : 0u;
+  for (uint64_t e = first; e < places; e += stride) {
+    const uint32_t t = targets[e];
+    new_targets[e] = t & hot_bit ? t : perm[t];
+  }
+  for (uint64_t h = first; h < hot_count; h += stride) new_hot[h] = perm[hot[h]];
+}
+
 static uint32_t grid_of(uint64_t items) {
   return (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(max_blocks(8), (items + 255) / 256));
 }
@@ -76,14 +91,17 @@ wc_status device_locality(wc_version* v, wc_error_detail* detail) {
   WC_TRY(c.targets.alloc(v->budget, m * 4 + kBulkPad, detail));
   if (v->weighted) WC_TRY(c.weights.alloc(v->budget, m * 8 + kBulkPad, detail));
   if (v->weighted && v->integral) WC_TRY(c.iweights.alloc(v->budget, m * 4 + kBulkPad, detail));
+  const LaneCsr& lanes = v->rev.lanes;
+  WC_TRY(L.lane_targets.alloc(v->budget, lanes.places * 4, detail));
+  if (lanes.hot_count) WC_TRY(L.lane_hot.alloc(v->budget, lanes.hot_count * 4, detail));
   if (n) {
-    // Order: a stable radix sort of (¬out-degree, id).
+    // Order: a stable radix sort of (¬length, id).
     DevBuf k0, k1, i1, temp;
     WC_TRY(k0.alloc(v->budget, n * 4, detail));
     WC_TRY(k1.alloc(v->budget, n * 4, detail));
     WC_TRY(i1.alloc(v->budget, n * 4, detail));
     note_launch(), degree_keys_kernel<<<grid_of(n), 256, 0, st>>>(
-        v->fwd.offsets.as<uint32_t>(), (uint32_t)n, k0.as<uint32_t>(), L.order.as<uint32_t>());
+        v->rev.offsets.as<uint32_t>(), (uint32_t)n, k0.as<uint32_t>(), L.order.as<uint32_t>());
     cub::DoubleBuffer<uint32_t> keys(k0.as<uint32_t>(), k1.as<uint32_t>());
     cub::DoubleBuffer<uint32_t> ids(L.order.as<uint32_t>(), i1.as<uint32_t>());
     size_t temp_bytes = 0;
@@ -116,6 +134,9 @@ wc_status device_locality(wc_version* v, wc_error_detail* detail) {
           v->rev.targets.as<uint32_t>(), v->weighted ? v->rev.weights.as<double>() : nullptr,
           c.iweights.ptr ? v->rev.iweights.as<int32_t>() : nullptr, c.offsets.as<uint32_t>(),
           (uint32_t)n, c.targets.as<uint32_t>(), c.weights.as<double>(), c.iweights.as<int32_t>());
+    note_launch(), loc_lanes_kernel<<<grid_of(lanes.places), 256, 0, st>>>(
+        lanes.targets.as<uint32_t>(), lanes.places, lanes.hot.as<uint32_t>(), lanes.hot_count,
+        L.perm.as<uint32_t>(), L.lane_targets.as<uint32_t>(), L.lane_hot.as<uint32_t>());
     WC_CUDA(cudaStreamSynchronize(st), detail);  // before the transient buffers go
   } else {
     WC_CUDA(cudaMemsetAsync(c.offsets.ptr, 0, 4, st), detail);

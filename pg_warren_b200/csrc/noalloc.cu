@@ -20,10 +20,6 @@
 
 namespace wc {
 
-wc_status prepare_pull(Ctx& ctx, DevCsr& csr, int semiring, int weighted_flag, int dtype,
-                       uint32_t width, PullLaunch& L);
-wc_status launch_pull(const PullLaunch& L, int dtype, const void* x, void* y);
-
 // The per-call working memory: 2n + 2n + n doubles (ranks, messages,
 // out-weights), the tombstone words, and the stop-test scalars.  64 MiB holds
 // a graph of about 1.67 million nodes at the default 100 iterations.
@@ -88,10 +84,8 @@ static wc_status static_setup(Ctx& ctx, PageRankRun& run, const wc_pagerank_opts
   WC_TRY((wc_status)sql_float<F_SUB>(1.0, o->damping, &teleport));
   if (o->has_tol && o->max_iter > 0)
     WC_TRY((wc_status)sql_float<F_MUL>(run.nodes, o->tol, &threshold));
-  run.local = true;  // wc_pagerank's own numbering, so the results are its
-  run.grid = pagerank_grid(run.csc(v));
-  run.long_grid = pagerank_long_grid(run.csc(v));
-  const uint32_t blocks = pagerank_partial_blocks(run.csc(v));  // block sums kept
+  run.grid = pagerank_grid(v->loc.csc);
+  const uint32_t blocks = pagerank_partial_blocks(v->loc.csc);  // block sums kept
 
   unsigned char* p = base;
   auto take = [&](uint64_t bytes) {
@@ -136,15 +130,11 @@ static wc_status static_setup(Ctx& ctx, PageRankRun& run, const wc_pagerank_opts
   s.iterations = reinterpret_cast<uint32_t*>(tail + 8);
   s.done = reinterpret_cast<int32_t*>(tail + 16);
   s.cancel = v->cancel_dev;
+  s.cancelled = reinterpret_cast<int32_t*>(tail + 24);
   s.pace = v->pace_dev;
   s.err = v->error.as<DeviceError>();
-  // out = plus_first over the forward CSR: each row's out-weight, into the
-  // second message buffer, then renumbered.
-  PullLaunch L;
-  WC_TRY(prepare_pull(ctx, v->fwd, WC_PLUS_FIRST, o->weighted, WC_F64, 1, L));
-  WC_TRY(launch_pull(L, WC_F64, x, s.msg[1]));
-  WC_TRY(to_locality(v, ctx.stream, s.msg[1], out));
-  return cuda_status(cudaGetLastError(), ctx.detail, "pagerank setup");
+  s.last_delta = reinterpret_cast<double*>(v->stage_dev + kStagePayload);
+  return run.out_weights(ctx);
 }
 
 // On an early return after work was queued on the call's stream, waits for

@@ -18,6 +18,7 @@
 // (documented; the ranks stay within 1e-12 relative L1).  The seeded
 // personalisation's sum is computed in the reference's own order (65536-
 // element chunks folded sequentially, combined in order).
+#include "lanes.cuh"
 #include "operand.h"
 #include "pagerank.h"
 #include "pull.cuh"
@@ -65,15 +66,15 @@ __device__ inline void block_sum_two(double& a, double& b) {
 // of them, then the block in fixed order), so the totals do not depend on
 // which block arrives last.  Returns true in thread 0 of that block, with
 // the totals in a, b.
-// `before`: block partials an earlier kernel of the same step stored at
-// the front of `partials` (added in, first).
+// `more(a, b)`: what each thread of the last block adds to its run of them.
+template <class More>
 __device__ inline bool reduce_two(double& a, double& b, double* partials, unsigned* counter,
-                                  unsigned before = 0) {
+                                  More more) {
   __shared__ bool last;
   block_sum_two(a, b);
   if (threadIdx.x == 0) {
-    partials[2 * (before + blockIdx.x)] = a;
-    partials[2 * (before + blockIdx.x) + 1] = b;
+    partials[2 * blockIdx.x] = a;
+    partials[2 * blockIdx.x + 1] = b;
     __threadfence();
     last = atomicAdd(counter, 1u) == gridDim.x - 1;
   }
@@ -81,16 +82,20 @@ __device__ inline bool reduce_two(double& a, double& b, double* partials, unsign
   if (!last) return false;
   __threadfence();
   double ta = 0.0, tb = 0.0;
-  for (unsigned k = threadIdx.x; k < before + gridDim.x; k += blockDim.x) {
+  for (unsigned k = threadIdx.x; k < gridDim.x; k += blockDim.x) {
     ta += __ldcg(partials + 2 * k);
     tb += __ldcg(partials + 2 * k + 1);
   }
+  more(ta, tb);
   block_sum_two(ta, tb);
   if (threadIdx.x != 0) return false;
   *counter = 0;
   a = ta;
   b = tb;
   return true;
+}
+__device__ inline bool reduce_two(double& a, double& b, double* partials, unsigned* counter) {
+  return reduce_two(a, b, partials, counter, [](double&, double&) {});
 }
 
 // The reference's sum of a seed over live rows (reduce.rs:137-153, 266-279):
@@ -153,14 +158,19 @@ __global__ void seed_shares_kernel(const double* seed, const uint64_t* tomb, uin
   }
 }
 
+__device__ __noinline__ void check_spread(double x, double out, DeviceError* err, uint32_t row) {
+  double m;
+  const int32_t s = sql_float<F_DIV>(x, out, &m);
+  if (s) raise(err, s, row);
+}
+
 // spread (mod.rs:204-232) for one row: the message, and the row's dangling
 // rank (x where out is not above 0 in SQL order).
 __device__ inline double spread_row(double x, double out, double* msg, DeviceError* err,
                                     uint32_t row) {
   if (sql_cmp_f(out, 0.0) > 0) {
-    double m;
-    int32_t s = sql_float<F_DIV>(x, out, &m);
-    if (s) raise(err, s, row);
+    const double m = x / out;
+    if (m == 0.0 || !isfinite(m)) check_spread(x, out, err, row);  // what a failing one leaves
     *msg = m;
     return 0.0;
   }
@@ -168,12 +178,23 @@ __device__ inline double spread_row(double x, double out, double* msg, DeviceErr
   return x;
 }
 
+// An unweighted row's out-weight is its entry count (the reference's sum of
+// that many ones), taken from the forward offsets here: the sum as a product
+// took 350 µs of a 5.9 ms solve on R-MAT 22.
 __global__ void pr_init_kernel(PrState s) {
   double none = 0.0, dangling = 0.0;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < s.n; i += gridDim.x * blockDim.x) {
     double x = tomb_at(s.tomb, i) ? 0.0 : s.start;
     s.x[0][i] = x;
-    dangling += spread_row(x, s.out[i], &s.msg[0][i], s.err, i);
+    double out;
+    if (s.degrees) {
+      const uint32_t id = __ldg(s.order + i);
+      out = (double)(s.degrees[id + 1] - s.degrees[id]);
+      s.out[i] = out;
+    } else {
+      out = s.out[i];
+    }
+    dangling += spread_row(x, out, &s.msg[0][i], s.err, i);
   }
   if (reduce_two(none, dangling, s.partials, s.counter)) {
     s.dangling[0] = dangling;
@@ -182,13 +203,33 @@ __global__ void pr_init_kernel(PrState s) {
   }
 }
 
+// A row's next rank by the reference's checked operations.
+__device__ __noinline__ double checked_next(double damping, double teleport, DeviceError* err,
+                                            uint32_t i, double y, double p, double dangling_in) {
+  double dp, flowed, a, b, next = 0.0;
+  int32_t e = sql_float<F_MUL>(dangling_in, p, &dp);
+  if (!e) e = sql_float<F_ADD>(y, dp, &flowed);
+  if (!e) e = sql_float<F_MUL>(damping, flowed, &a);
+  if (!e) e = sql_float<F_MUL>(teleport, p, &b);
+  if (!e) e = sql_float<F_ADD>(a, b, &next);
+  if (e) raise(err, e, i);
+  return next;
+}
+
 // advance (mod.rs:245-282) and the next spread, for the row the pull ends.
 struct PrEpi {
   const PrState* s;
   int cur;
   double dangling_in;
-  double delta;
-  double dangling_out;
+  double delta = 0.0;
+  double dangling_out = 0.0;
+  // dangling · start and teleport · start, and whether neither failed.
+  double uniform_dp = 0.0, uniform_b = 0.0;
+  bool uniform_ok = false;
+  __device__ PrEpi(const PrState* st, int c, double in) : s(st), cur(c), dangling_in(in) {
+    uniform_ok = sql_float<F_MUL>(in, st->start, &uniform_dp) == 0 &&
+                 sql_float<F_MUL>(st->teleport, st->start, &uniform_b) == 0;
+  }
   // The row's operands, requested before its pull so they arrive with it.
   struct Pre {
     double old, out, share;
@@ -203,28 +244,44 @@ struct PrEpi {
     p.out = st.out[i];
     return p;
   }
-  __device__ void row(uint32_t i, bool present, double y, const Pre& pr) {
+  typedef Partial<double, semiring_add(WC_PLUS_TIMES)> Slot;
+  // With the uniform personalisation two of the products are the launch's.
+  // Every failing operation leaves an infinity, a NaN or a zero product, so
+  // only a row that shows one goes through the checked operations.  A row
+  // finished by whichever warp came last leaves its share of the sums in its
+  // slot, for the last block to add in row order.
+  __device__ void row(uint32_t i, bool present, double y, const Pre& pr, Slot* slot = nullptr) {
     const PrState& st = *s;
     if (!present) y = 0.0;  // an empty row writes the plus identity
-    double next = 0.0;
-    if (!pr.dead) {
-      const double p = pr.share;
-      double dp, flowed, a, b;
-      int32_t e = sql_float<F_MUL>(dangling_in, p, &dp);
-      if (!e) e = sql_float<F_ADD>(y, dp, &flowed);
-      if (!e) e = sql_float<F_MUL>(st.damping, flowed, &a);
-      if (!e) e = sql_float<F_MUL>(st.teleport, p, &b);
-      if (!e) e = sql_float<F_ADD>(a, b, &next);
-      if (e) raise(st.err, e, i);
-    }
-    delta += fabs(next - pr.old);
+    const double flowed = st.damping * (y + uniform_dp);
+    double next = flowed + uniform_b;
+    if (pr.dead)
+      next = 0.0;
+    else if (st.shares || flowed == 0.0 || !isfinite(next) || !uniform_ok)
+      next = checked_next(st.damping, st.teleport, st.err, i, y, pr.share, dangling_in);
+    const double change = fabs(next - pr.old);
     st.x[cur ^ 1][i] = next;
-    dangling_out += spread_row(next, pr.out, &st.msg[cur ^ 1][i], st.err, i);
+    const double dangles = spread_row(next, pr.out, &st.msg[cur ^ 1][i], st.err, i);
+    if (slot) {
+      static_assert(sizeof(Slot) == sizeof(double2), "a slot holds the row's two sums");
+      *reinterpret_cast<double2*>(slot) = make_double2(change, dangles);
+    } else {
+      delta += change;
+      dangling_out += dangles;
+    }
   }
 };
 
-// Unweighted, four blocks an SM (64 registers) keep more gathers in flight;
-// with weights the extra registers would spill, so three.
+// The caller's cancel word (host memory, mapped), requested by one thread of
+// an iteration as it begins and passed to the device's copy as it ends, so the
+// round trip over PCIe runs beside the iteration.
+__device__ inline int32_t pr_read_cancel(const PrState& s) {
+  return blockIdx.x == 0 && threadIdx.x == 32 ? *(volatile const int32_t*)s.cancel : 0;
+}
+__device__ inline void pr_pass_cancel(const PrState& s, int32_t cancel) {
+  if (blockIdx.x == 0 && threadIdx.x == 32) *(volatile int32_t*)s.cancelled = cancel;
+}
+
 // The step's close, by the last block of its last kernel: the stop test,
 // the cancel word and the progress words.
 __device__ inline void pr_close(const PrState& s, uint32_t it, double delta, double dangling) {
@@ -232,104 +289,108 @@ __device__ inline void pr_close(const PrState& s, uint32_t it, double delta, dou
   s.dangling[it + 1] = dangling;
   *s.iterations = it + 1;
   if (s.has_tol && sql_cmp_f(delta, s.threshold) < 0) *s.done = 1;
-  // The caller's cancel word (host memory, mapped) is read once per
-  // iteration, here; the next iteration then returns at once.
-  if (*(volatile const int32_t*)s.cancel) {
+  // The caller's cancel word was read once, as the iteration began; the next
+  // iteration then returns at once.
+  if (*(volatile const int32_t*)s.cancelled) {
     raise(s.err, WC_CANCELLED);
     *s.done = 1;
   }
   // Tell the host how far the solve is, so it stops queueing iterations.
   if (s.pace) {
+    *(volatile double*)s.last_delta = delta;
     volatile uint32_t* pace = s.pace;
     pace[1] = *s.done;
     pace[0] = it + 1;
   }
 }
 
-// DEFER: the long rows' pieces only store their partials, and
-// pr_long_kernel finishes those rows and the step; each block here leaves
-// its sums at the front of the partials.
-template <class W, bool SPLIT, bool DEFER>
+// The reverse CSR's lane-major copy with its targets in the sorted numbering:
+// a slice's rows are consecutive there, so the epilogue's vectors are read and
+// written in runs (by dense id they took 32-byte sectors apiece, which cost
+// as much again as the gathers: 702 against 465 µs for the product alone).
+template <class W> static LaneView<W> ranked_view(const PullLaunch& L, const wc_version* v) {
+  LaneView<W> A = lane_view<W>(L);
+  A.rows = nullptr;
+  A.first_short = v->rev.schedule.long_rows;
+  A.numbers = v->loc.perm.as<uint32_t>();
+  A.tgt = v->loc.lane_targets.as<uint32_t>();
+  A.hot = v->loc.lane_hot.as<uint32_t>();
+  return A;
+}
+
+// One iteration over the reverse CSR's lane-major copy: one launch, one
+// block an SM.
+template <class W>
+__global__ void __launch_bounds__(kLaneThreads, 1)
+    pr_lane_kernel(LaneView<W> A, PrState s, uint32_t it, const uint4* longs, uint32_t long_count,
+                   uint32_t run) {
+  extern __shared__ __align__(16) double pr_hot[];
+  const int cur = it & 1;
+  const int32_t done = *(volatile int32_t*)s.done;
+  const int32_t cancel = pr_read_cancel(s);
+  PrEpi epi(&s, cur, s.dangling[it]);
+  lane_fill_hot<double, W>(A, s.msg[cur], pr_hot);
+  if (done) return;
+  lane_units<double, WC_PLUS_TIMES, W>(A, s.msg[cur], pr_hot, epi, s.err);
+  pr_pass_cancel(s, cancel);
+  double delta = epi.delta, dangling = epi.dangling_out;
+  // The rows of several units left their shares of the sums in their slots.
+  auto more = [&](double& a, double& b) {
+    for (uint32_t r = threadIdx.x; r < long_count; r += blockDim.x) {
+      const uint4 L = __ldg(longs + r);  // row, first slot, pieces
+      if (L.z <= run) continue;
+      const double2 v = __ldcg(reinterpret_cast<const double2*>(
+          static_cast<const PrEpi::Slot*>(A.carry) + L.y));
+      a += v.x;
+      b += v.y;
+    }
+  };
+  if (reduce_two(delta, dangling, s.partials, s.counter, more)) pr_close(s, it, delta, dangling);
+}
+
+// One iteration over a range of the row-split schedule of the
+// locality-ordered CSC (a part of a row-partitioned solve).  Unweighted, four
+// blocks an SM (64 registers) keep more gathers in flight; with weights the
+// extra registers would spill, so three.
+template <class W>
 __global__ void __launch_bounds__(kPullThreads, WSize<W>::v == 0 ? 4 : 3)
     pr_iter_kernel(CsrView<W> A, PrState s, uint32_t it) {
   extern __shared__ __align__(16) unsigned char smem[];
   if (*(volatile int32_t*)s.done) return;
+  const int32_t cancel = pr_read_cancel(s);
   const int cur = it & 1;
-  PrEpi epi{&s, cur, s.dangling[it], 0.0, 0.0};
+  PrEpi epi(&s, cur, s.dangling[it]);
   PullRing<double, W>* ring = reinterpret_cast<PullRing<double, W>*>(smem) + (threadIdx.x >> 5);
-  pull_units<double, WC_PLUS_TIMES, W, PrEpi, SPLIT, DEFER>(A, s.msg[cur], epi, s.err, ring);
+  pull_units<double, WC_PLUS_TIMES, W>(A, s.msg[cur], epi, s.err, ring);
+  pr_pass_cancel(s, cancel);
   double delta = epi.delta, dangling = epi.dangling_out;
-  if constexpr (DEFER) {
-    block_sum_two(delta, dangling);
-    if (threadIdx.x == 0) {
-      s.partials[2 * blockIdx.x] = delta;
-      s.partials[2 * blockIdx.x + 1] = dangling;
-    }
-    return;
-  }
   if (reduce_two(delta, dangling, s.partials, s.counter)) pr_close(s, it, delta, dangling);
 }
 
-// The long rows of a step run with DEFER: a warp per row combines its
-// pieces' partials in piece order (as the last piece to arrive does
-// otherwise), then the row's advance and spread; the last block reduces
-// both kernels' block sums in a fixed order and closes the step.
-__global__ void __launch_bounds__(256)
-    pr_long_kernel(const uint4* longs, uint32_t long_count,
-                   const Partial<double, semiring_add(WC_PLUS_TIMES)>* carry, PrState s,
-                   uint32_t it, uint32_t first_blocks) {
-  if (*(volatile int32_t*)s.done) return;
-  const int cur = it & 1;
-  PrEpi epi{&s, cur, s.dangling[it], 0.0, 0.0};
-  const unsigned lane = threadIdx.x & 31;
-  const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-  for (uint32_t r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < long_count; r += warps) {
-    const uint4 L = longs[r];  // row, first slot, pieces
-    PrEpi::Pre pre{};
-    if (lane == 0) pre = epi.pre(L.x);
-    const auto total =
-        combine_pieces<double, semiring_add(WC_PLUS_TIMES), 1>(carry, L.y, L.z, 0, lane);
-    if (lane == 0) {
-      double v;
-      const int32_t st = total.acc.value(&v);
-      if (st) raise(s.err, st, L.x);
-      epi.row(L.x, true, v, pre);
-    }
-  }
-  double delta = epi.delta, dangling = epi.dangling_out;
-  if (reduce_two(delta, dangling, s.partials, s.counter, first_blocks))
-    pr_close(s, it, delta, dangling);
+template <class W>
+static wc_status launch_iter(const PullLaunch& L, const PrState& s, uint32_t it, uint32_t blocks,
+                             const wc_version* v) {
+  const Schedule& longs = v->rev.schedule;
+  static const cudaError_t attr =
+      cudaFuncSetAttribute(pr_lane_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)(kHotSlots * sizeof(double)));
+  if (attr != cudaSuccess) return cuda_status(attr, L.detail, "pagerank kernel attributes");
+  const LaneView<W> A = ranked_view<W>(L, v);
+  note_launch(), pr_lane_kernel<W><<<blocks, kLaneThreads, A.hot_count * sizeof(double),
+                                     L.stream>>>(A, s, it, longs.long_list.as<uint4>(),
+                                                 longs.long_rows, L.lanes->run);
+  return WC_OK;
 }
 
-template <class W, bool SPLIT, bool DEFER>
-static wc_status set_iter_attributes(const PullLaunch& L) {
+template <class W>
+static wc_status launch_part(const PullLaunch& L, const PrState& s, uint32_t it, uint32_t blocks) {
+  CsrView<W> A{L.off, L.tgt, static_cast<const W*>(L.weights), L.units, L.unit_count, L.counters,
+               L.carry};
   constexpr size_t smem = pull_smem_bytes<double, W>();
   static const cudaError_t attr = cudaFuncSetAttribute(
-      pr_iter_kernel<W, SPLIT, DEFER>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  return cuda_status(attr, L.detail, "pagerank kernel attributes");
-}
-
-// One iteration: pr_iter_kernel over L's units, and with `longs` (the
-// schedule's long rows, DEFER) pr_long_kernel after it on `long_grid` blocks.
-template <class W>
-wc_status launch_iter(const PullLaunch& L, const PrState& s, uint32_t it, uint32_t blocks,
-                      const Schedule* longs = nullptr, uint32_t long_grid = 0) {
-  CsrView<W> A{L.off, L.tgt, static_cast<const W*>(L.weights), L.units, L.unit_count, L.counters,
-               L.carry, L.hot};
-  constexpr size_t smem = pull_smem_bytes<double, W>();
-  if (longs) {
-    WC_TRY((set_iter_attributes<W, true, true>(L)));
-    note_launch(), pr_iter_kernel<W, true, true><<<blocks, kPullThreads, smem, L.stream>>>(A, s, it);
-    note_launch(), pr_long_kernel<<<long_grid, 256, 0, L.stream>>>(
-        longs->long_list.as<uint4>(), longs->long_rows,
-        static_cast<const Partial<double, semiring_add(WC_PLUS_TIMES)>*>(L.carry), s, it, blocks);
-  } else if (L.hot) {
-    WC_TRY((set_iter_attributes<W, true, false>(L)));
-    note_launch(), pr_iter_kernel<W, true, false><<<blocks, kPullThreads, smem, L.stream>>>(A, s, it);
-  } else {
-    WC_TRY((set_iter_attributes<W, false, false>(L)));
-    note_launch(), pr_iter_kernel<W, false, false><<<blocks, kPullThreads, smem, L.stream>>>(A, s, it);
-  }
+      pr_iter_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (attr != cudaSuccess) return cuda_status(attr, L.detail, "pagerank kernel attributes");
+  note_launch(), pr_iter_kernel<W><<<blocks, kPullThreads, smem, L.stream>>>(A, s, it);
   return WC_OK;
 }
 
@@ -344,8 +405,8 @@ wc_status launch_pr_init(const PrState& s, uint32_t grid, cudaStream_t stream) {
 
 wc_status launch_part_iteration(const PullLaunch& L, const PrState& s, uint32_t it,
                                 uint32_t blocks) {
-  if (L.weight_kind == WEIGHTS_F64) return launch_iter<double>(L, s, it, blocks);
-  return launch_iter<void>(L, s, it, blocks);
+  if (L.weight_kind == WEIGHTS_F64) return launch_part<double>(L, s, it, blocks);
+  return launch_part<void>(L, s, it, blocks);
 }
 
 uint64_t live_count(const uint64_t* tomb, uint64_t n) {
@@ -359,12 +420,11 @@ uint64_t live_count(const uint64_t* tomb, uint64_t n) {
   return n - dead;
 }
 
-uint32_t pagerank_long_grid(const DevCsr& csc) {
-  return std::max<uint32_t>(1, std::min<uint32_t>((csc.schedule.long_rows + 7) / 8, max_blocks(2)));
-}
-
+// The sums of pagerank_grid blocks, and room that the working memory of
+// wc_pagerank_noalloc has always counted beside them.
 uint32_t pagerank_partial_blocks(const DevCsr& csc) {
-  return pagerank_grid(csc) + pagerank_long_grid(csc);
+  return pagerank_grid(csc) +
+         std::max<uint32_t>(1, std::min<uint32_t>((csc.schedule.long_rows + 7) / 8, max_blocks(2)));
 }
 
 uint32_t pagerank_grid(const DevCsr& csc) {
@@ -373,12 +433,11 @@ uint32_t pagerank_grid(const DevCsr& csc) {
 }
 
 wc_status PageRankRun::setup(Ctx& ctx, const wc_pagerank_opts* o, const uint64_t* tomb_host,
-                             const double* seed, bool in_locality_order) {
+                             const double* seed) {
   wc_version* v = ctx.v;
   const uint64_t n = v->n;
   const uint64_t words = (n + 63) / 64;
   opts = *o;
-  local = in_locality_order;
   // Tombstones: the caller's words, on the device.
   std::vector<uint64_t> host_words;
   const uint64_t* th = tomb_host;
@@ -396,10 +455,8 @@ wc_status PageRankRun::setup(Ctx& ctx, const wc_pagerank_opts* o, const uint64_t
   WC_TRY((wc_status)sql_float<F_SUB>(1.0, o->damping, &teleport));
   double threshold = 0.0;
   if (o->has_tol && o->max_iter > 0) WC_TRY((wc_status)sql_float<F_MUL>(nodes, o->tol, &threshold));
-  const uint32_t blocks = pagerank_grid(csc(v));
-  grid = blocks;
-  long_grid = pagerank_long_grid(csc(v));
-  const uint32_t partial_blocks = blocks + long_grid;
+  grid = pagerank_grid(v->loc.csc);
+  const uint32_t partial_blocks = pagerank_partial_blocks(v->loc.csc);
   WC_TRY(ctx.scratch(POOL_PR_X, 2 * n * 8, &x));
   WC_TRY(ctx.scratch(POOL_PR_MSG, 2 * n * 8, &msg));
   WC_TRY(ctx.scratch(POOL_PR_OUT, n * 8, &out));
@@ -407,15 +464,13 @@ wc_status PageRankRun::setup(Ctx& ctx, const wc_pagerank_opts* o, const uint64_t
   WC_TRY(ctx.scratch(POOL_PR_SCALARS, scalar_bytes, &scalars));
   uint64_t* tomb_dev = nullptr;
   if (th) {
-    // In locality order the words are renumbered into the buffer's second half.
-    WC_TRY(ctx.scratch(POOL_PR_TOMB, words * 8 * (local ? 2 : 1), &tomb));
+    // The words are renumbered into the buffer's second half.
+    WC_TRY(ctx.scratch(POOL_PR_TOMB, words * 8 * 2, &tomb));
     WC_CUDA(cudaMemcpyAsync(tomb->ptr, th, words * 8, cudaMemcpyHostToDevice, ctx.stream),
             ctx.detail);
     tomb_dev = tomb->as<uint64_t>();
-    if (local) {
-      WC_TRY(bits_to_locality(v, ctx.stream, tomb_dev, tomb_dev + words));
-      tomb_dev += words;
-    }
+    WC_TRY(bits_to_locality(v, ctx.stream, tomb_dev, tomb_dev + words));
+    tomb_dev += words;
   }
   WC_CUDA(cudaMemsetAsync(scalars->ptr, 0, scalar_bytes, ctx.stream), ctx.detail);
   double* sc = scalars->as<double>();
@@ -440,42 +495,66 @@ wc_status PageRankRun::setup(Ctx& ctx, const wc_pagerank_opts* o, const uint64_t
   s.iterations = reinterpret_cast<uint32_t*>(tail + 8);
   s.done = reinterpret_cast<int32_t*>(tail + 16);
   s.cancel = v->cancel_dev;
+  s.cancelled = reinterpret_cast<int32_t*>(tail + 24);
   s.pace = v->pace_dev;
   s.err = v->error.as<DeviceError>();
-  // out = plus_first over the forward CSR: each row's out-weight (in
-  // locality order: into the second message buffer, then renumbered).
-  PullLaunch L;
-  WC_TRY(prepare_pull(ctx, v->fwd, WC_PLUS_FIRST, o->weighted, WC_F64, 1, L));
-  WC_TRY(launch_pull(L, WC_F64, s.x[0], local ? s.msg[1] : out->ptr));
-  if (local) WC_TRY(to_locality(v, ctx.stream, s.msg[1], out->as<double>()));
+  s.last_delta = reinterpret_cast<double*>(v->stage_dev + kStagePayload);
+  WC_TRY(out_weights(ctx));
   // The personalisation, summed in dense-id order (the reference's chunks).
   if (seed) {
     Operand S(POOL_SEED);
     WC_TRY(S.in(ctx, seed, n * 8));
     const double* sd = static_cast<const double*>(S.dev);
     const uint32_t chunks = (uint32_t)((n + kChunk - 1) / kChunk);
-    WC_TRY(ctx.scratch(POOL_PR_SHARES, n * 8 * (local ? 2 : 1) + (uint64_t)chunks * 8, &shares));
-    double* partial = shares->as<double>() + n * (local ? 2 : 1);
+    WC_TRY(ctx.scratch(POOL_PR_SHARES, n * 8 * 2 + (uint64_t)chunks * 8, &shares));
+    double* partial = shares->as<double>() + n * 2;
     const uint64_t* tomb_ids = th ? tomb->as<uint64_t>() : nullptr;  // dense-id order
     if (chunks)
       note_launch(), seed_chunks_kernel<<<chunks, 256, 0, ctx.stream>>>(sd, tomb_ids, n, partial);
     note_launch(), seed_shares_kernel<<<max_blocks(4), 256, 0, ctx.stream>>>(sd, tomb_ids, (uint32_t)n, partial,
                                                              chunks, shares->as<double>(), s.err);
-    s.shares = shares->as<double>();
-    if (local) {
-      WC_TRY(to_locality(v, ctx.stream, shares->as<double>(), shares->as<double>() + n));
-      s.shares = shares->as<double>() + n;
-    }
+    WC_TRY(to_locality(v, ctx.stream, shares->as<double>(), shares->as<double>() + n));
+    s.shares = shares->as<double>() + n;
   }
   return cuda_status(cudaGetLastError(), ctx.detail, "pagerank setup");
+}
+
+// The out-weights, s.out: plus_first over the forward CSR when weighted
+// (renumbered through the second message buffer); when not, the rows' entry
+// counts, which pr_init_kernel takes from the offsets.
+wc_status PageRankRun::out_weights(Ctx& ctx) {
+  wc_version* v = ctx.v;
+  if (opts.weighted == 0 || !v->weighted) {
+    s.degrees = v->fwd.offsets.as<uint32_t>();
+    s.order = v->loc.order.as<uint32_t>();
+    return WC_OK;
+  }
+  PullLaunch L;
+  WC_TRY(prepare_pull(ctx, v->fwd, WC_PLUS_FIRST, opts.weighted, WC_F64, 1, L));
+  WC_TRY(launch_pull(L, WC_F64, s.x[0], s.msg[1]));
+  return to_locality(v, ctx.stream, s.msg[1], s.out);
+}
+
+__global__ void out_degrees_kernel(PrState s) {
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < s.n; i += gridDim.x * blockDim.x) {
+    const uint32_t id = __ldg(s.order + i);
+    s.out[i] = (double)(s.degrees[id + 1] - s.degrees[id]);
+  }
+}
+
+wc_status PageRankRun::out_now(Ctx& ctx) {
+  if (s.degrees && s.n)
+    note_launch(), out_degrees_kernel<<<max_blocks(4), 256, 0, ctx.stream>>>(s);
+  return cuda_status(cudaGetLastError(), ctx.detail, "out-degrees");
 }
 
 wc_status PageRankRun::run(Ctx& ctx) {
   wc_version* v = ctx.v;
   WC_TRY(launch_pr_init(s, grid, ctx.stream));
   PullLaunch L;
-  WC_TRY(prepare_pull(ctx, const_cast<DevCsr&>(csc(v)), WC_PLUS_TIMES, opts.weighted, WC_F64, 1, L));
-  if (local) L.hot = kPageRankHotNodes;
+  WC_TRY(prepare_pull(ctx, v->rev, WC_PLUS_TIMES, opts.weighted, WC_F64, 1, L));
+  // No more blocks than the step keeps sums for.
+  const uint32_t blocks = L.lanes ? std::min(lane_grid(L), grid) : 0;
   // With a tolerance the solve usually stops well before max_iter: the
   // host keeps at most kAhead iterations queued beyond the last one the
   // device reported, and stops queueing once the device reports the stop,
@@ -487,7 +566,7 @@ wc_status PageRankRun::run(Ctx& ctx) {
     pace[1] = 0;
   }
   ctx.phase_begin("iteration");
-  for (uint32_t it = 0; it < opts.max_iter; it++) {
+  for (uint32_t it = 0; L.lanes && it < opts.max_iter; it++) {
     // A cancel stops the queueing (the kernels queued read the device's
     // copy of the word, which finish() raises).
     if (ctx.cancelled()) break;
@@ -499,11 +578,8 @@ wc_status PageRankRun::run(Ctx& ctx) {
       }
       if (stop) break;
     }
-    // In the locality order the long rows are finished by a pass of their
-    // own, after their pieces (no release/acquire arrival per piece).
-    const Schedule* longs = local ? &csc(v).schedule : nullptr;
-    if (L.weight_kind == WEIGHTS_F64) WC_TRY(launch_iter<double>(L, s, it, grid, longs, long_grid));
-    else WC_TRY(launch_iter<void>(L, s, it, grid, longs, long_grid));
+    if (L.weight_kind == WEIGHTS_F64) WC_TRY(launch_iter<double>(L, s, it, blocks, v));
+    else WC_TRY(launch_iter<void>(L, s, it, blocks, v));
   }
   ctx.phase_end();
   return cuda_status(cudaGetLastError(), ctx.detail, "pagerank iterations");
@@ -511,22 +587,24 @@ wc_status PageRankRun::run(Ctx& ctx) {
 
 wc_status PageRankRun::result(Ctx& ctx, double* ranks_dev_or_host, uint32_t* iterations_out,
                               double* margin) {
+  // A solve that reported its progress left the count and the last change in
+  // mapped memory, complete once finish() has waited.
   uint32_t its = 0;
-  WC_CUDA(cudaMemcpy(&its, s.iterations, 4, cudaMemcpyDeviceToHost), ctx.detail);
+  if (s.pace) its = ctx.v->pace_host[0];
+  else WC_CUDA(cudaMemcpy(&its, s.iterations, 4, cudaMemcpyDeviceToHost), ctx.detail);
   if (opts.max_iter == 0) its = 0;
   const double* final_x = s.x[its & 1];
-  if (local) {
-    // Back to dense-id order, through the other rank buffer (free now).
-    WC_TRY(from_locality(ctx.v, ctx.stream, final_x, s.x[(its & 1) ^ 1]));
-    final_x = s.x[(its & 1) ^ 1];
-  }
+  // Back to dense-id order, through the other rank buffer (free now).
+  WC_TRY(from_locality(ctx.v, ctx.stream, final_x, s.x[(its & 1) ^ 1]));
+  final_x = s.x[(its & 1) ^ 1];
   WC_CUDA(cudaMemcpyAsync(ranks_dev_or_host, final_x, ctx.v->n * 8, cudaMemcpyDefault, ctx.stream),
           ctx.detail);
   WC_CUDA(cudaStreamSynchronize(ctx.stream), ctx.detail);
   if (iterations_out) *iterations_out = its;
   if (margin && its > 0) {
     double delta = 0.0;
-    WC_CUDA(cudaMemcpy(&delta, s.delta + (its - 1), 8, cudaMemcpyDeviceToHost), ctx.detail);
+    if (s.pace) std::memcpy(&delta, ctx.v->stage_host + kStagePayload, 8);
+    else WC_CUDA(cudaMemcpy(&delta, s.delta + (its - 1), 8, cudaMemcpyDeviceToHost), ctx.detail);
     *margin = s.threshold != 0.0 ? delta / s.threshold : 0.0;
   }
   return WC_OK;
@@ -548,7 +626,7 @@ wc_status wc_pagerank(wc_version* v, const wc_call* call, const wc_pagerank_opts
   WC_TRY(ctx.begin());
   PageRankRun run;
   ctx.phase_begin("setup");
-  WC_TRY(run.setup(ctx, o, tombstones, o->seed, true));
+  WC_TRY(run.setup(ctx, o, tombstones, o->seed));
   ctx.phase_end();
   ctx.progress("iterating", 0, o->max_iter);
   WC_TRY(run.run(ctx));

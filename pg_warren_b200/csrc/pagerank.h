@@ -11,7 +11,9 @@ struct PrState {
   uint32_t n;
   double* x[2];
   double* msg[2];
-  const double* out;
+  double* out;
+  const uint32_t* degrees;  // unweighted: the forward offsets pr_init takes `out` from
+  const uint32_t* order;    //   by the rows' dense ids; else NULL
   const double* shares;  // NULL: uniform, `start` at every live row
   const uint64_t* tomb;
   double start, damping, teleport, threshold;
@@ -22,8 +24,10 @@ struct PrState {
   unsigned* counter;
   uint32_t* iterations;
   int32_t* done;
-  const int32_t* cancel;
+  const int32_t* cancel;  // the caller's word, host-mapped
+  int32_t* cancelled;     // what an iteration read there as it began
   uint32_t* pace;  // host-mapped: [0] iterations done, [1] stopped
+  double* last_delta;  // host-mapped: the last iteration's change (with `pace`)
   DeviceError* err;
 };
 
@@ -32,27 +36,20 @@ struct PageRankRun {
   uint64_t live = 0;
   double nodes = 0.0;
   uint32_t grid = 1;
-  uint32_t long_grid = 1;  // pr_long_kernel's blocks (locality order)
-  // The solve pulls over the version's locality-ordered CSC (v->loc), its
-  // vectors in that numbering; inputs are renumbered in by setup and the
-  // ranks out by result.  Off for callers that read the vectors themselves.
-  bool local = false;
+  // The vectors are numbered as the version's CSC in row order (v->loc):
+  // setup renumbers its inputs in and result the ranks out.
   DevBuf *x = nullptr, *msg = nullptr, *out = nullptr, *shares = nullptr, *tomb = nullptr,
          *scalars = nullptr;
   PrState s;
 
   wc_status setup(Ctx& ctx, const wc_pagerank_opts* o, const uint64_t* tomb_host,
-                  const double* seed, bool in_locality_order = false);
-  // The CSC the iterations pull over and the grid for it.
-  const DevCsr& csc(const wc_version* v) const { return local ? v->loc.csc : v->rev; }
+                  const double* seed);
+  wc_status out_weights(Ctx& ctx);
+  // s.out by itself, for a caller that does not run pr_init_kernel.
+  wc_status out_now(Ctx& ctx);
   wc_status run(Ctx& ctx);
   wc_status result(Ctx& ctx, double* ranks, uint32_t* iterations, double* margin);
 };
-
-// Over the locality-ordered CSC, the messages of the nodes numbered below
-// this (the most gathered) are kept in L1: 64 KB of them, what the SM's L1
-// holds beside four blocks' staging rings.
-constexpr uint32_t kPageRankHotNodes = 8192;
 
 uint64_t live_count(const uint64_t* tomb, uint64_t n);
 // pr_init_kernel: the start vector, its messages and dangling rank.
@@ -66,10 +63,8 @@ void pagerank_part_forget(const wc_version* v);
 // The row-partitioned search's and product's state kept with a version
 // (bfs_part.cu), dropped when the version is released.
 void bfs_part_forget(const wc_version* v);
-// Blocks of an iteration launch over `csc`; of the long-row pass that
-// follows it in the locality order; and the block sums the step keeps.
+// Blocks of an iteration launch over `csc`, and the block sums kept for it.
 uint32_t pagerank_grid(const DevCsr& csc);
-uint32_t pagerank_long_grid(const DevCsr& csc);
 uint32_t pagerank_partial_blocks(const DevCsr& csc);
 
 }  // namespace wc

@@ -161,7 +161,7 @@ wc_status wc_pagerank_part_begin(wc_version* v, const wc_call* call, const wc_pa
   ps->unit_begin = uc[part];
   ps->unit_end = uc[part + 1];
   PageRankRun& run = ps->run;
-  WC_TRY(run.setup(ctx, o, tombstones, nullptr, true));
+  WC_TRY(run.setup(ctx, o, tombstones, nullptr));
   // The rank and message vectors are the caller's (it exchanges their rows).
   const uint64_t n = v->n;
   run.s.x[0] = ranks2;
@@ -205,7 +205,6 @@ wc_status wc_pagerank_part_step(wc_version* v, const wc_call* call, uint32_t ite
   WC_TRY(prepare_pull(ctx, v->loc.csc, WC_PLUS_TIMES, run.opts.weighted, WC_F64, 1, L));
   L.units += ps->unit_begin;
   L.unit_count = ps->unit_end - ps->unit_begin;
-  L.hot = kPageRankHotNodes;
   if (L.unit_count) WC_TRY(launch_part_iteration(L, run.s, iteration, run.grid));
   WC_TRY(ctx.finish());
   double host[2] = {0.0, 0.0};

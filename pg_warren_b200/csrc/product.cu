@@ -46,11 +46,14 @@ wc_status prepare_pull(Ctx& ctx, DevCsr& csr, int semiring, int weighted_flag, i
     if (dtype == WC_I64 && v->integral) {
       L.weight_kind = WEIGHTS_I32;
       L.weights = csr.iweights.ptr;
+      L.lane_weights = csr.lanes.iweights.ptr;
     } else {
       L.weight_kind = WEIGHTS_F64;
       L.weights = csr.weights.ptr;
+      L.lane_weights = csr.lanes.weights.ptr;
     }
   }
+  L.lanes = csr.lanes.count || csr.lanes.shorts ? &csr.lanes : nullptr;
   L.units = csr.schedule.units.as<Unit>();
   L.unit_count = csr.schedule.count;
   L.counters = csr.schedule.counters.as<uint32_t>();
@@ -120,6 +123,7 @@ static wc_status product(wc_version* v, const wc_call* call, const wc_product* p
     WC_TRY(schedule_part_cuts(v, csr, parts, uc, rc, ctx.detail));
     L.units += uc[part];
     L.unit_count = uc[part + 1] - uc[part];
+    L.lanes = nullptr;  // a range of the rows: over the row-split schedule
   }
   if (width > 1) {
     DevBuf* mc;

@@ -41,7 +41,10 @@ struct PullLaunch {
   DeviceError* err;
   wc_error_detail* detail;
   WriteArgs write;
-  uint32_t hot;  // over a locality-ordered CSC: gathers of j < hot kept in L1 (0: none)
+  // The orientation's lane-major copy and its weights as `weight_kind` says
+  // (NULL: none, or a part of the rows only: the row-split schedule is walked).
+  const LaneCsr* lanes;
+  const void* lane_weights;
 };
 
 // Cuts `csr`'s schedule into `parts` ranges of about equal entries at unit

@@ -32,9 +32,6 @@ constexpr int kPullWarps = kPullThreads / 32;
 
 // One CSR orientation as the kernels read it.  W: double (f64 weights),
 // int32_t (the integral copy) or void (unweighted: every weight 1).
-// `hot`: over a locality-ordered CSC (nodes numbered by out-degree, largest
-// first), the gathers of x_j with j < hot are kept in L1 and the others
-// bypass it; 0 for a CSC in dense-id order (every gather as any other).
 template <class W> struct CsrView {
   const uint32_t* off;
   const uint32_t* tgt;
@@ -43,7 +40,6 @@ template <class W> struct CsrView {
   uint32_t unit_count;
   uint32_t* counters;
   void* carry;
-  uint32_t hot = 0;
 };
 template <> struct CsrView<void> {
   const uint32_t* off;
@@ -53,7 +49,6 @@ template <> struct CsrView<void> {
   uint32_t unit_count;
   uint32_t* counters;
   void* carry;
-  uint32_t hot = 0;
 };
 
 // An entry's weight as stored (WT), loaded apart from its product so the
@@ -89,28 +84,6 @@ template <class E, int S> struct EntryOf<E, S, void> {
 template <class E> __device__ inline E load_x(const E* x, uint32_t j) { return __ldg(x + j); }
 template <> __device__ inline bool8 load_x<bool8>(const bool8* x, uint32_t j) {
   return *(x + j);
-}
-
-// A gather over a locality-ordered CSC: the few most gathered values (j <
-// hot) are kept in L1, the rest are read past it so they do not evict those;
-// in L2 every value is kept ahead of the streamed CSR (`keep`: an
-// l2_evict_last_policy).  8-byte elements only; others take load_x.
-template <class E>
-__device__ inline E load_x_split(const E* x, uint32_t j, uint32_t hot, uint64_t keep) {
-  if constexpr (sizeof(E) == 8) {
-    unsigned long long b;
-    if (j < hot)
-      asm("ld.global.nc.L1::evict_last.L2::cache_hint.b64 %0, [%1], %2;"
-          : "=l"(b) : "l"(x + j), "l"(keep));
-    else
-      asm("ld.global.nc.L1::no_allocate.L2::cache_hint.b64 %0, [%1], %2;"
-          : "=l"(b) : "l"(x + j), "l"(keep));
-    E v;
-    memcpy(&v, &b, 8);
-    return v;
-  } else {
-    return load_x(x, j);
-  }
 }
 
 // An accumulator with a presence flag: the first entry sets the sum.
@@ -253,26 +226,18 @@ __device__ inline typename EntryOf<E, S, W>::WT ring_weight(const PullRing<E, W>
 // Stages the products of the unit in buffer b (count <= 256 entries) in the
 // warp's stage: each lane gathers its (up to 8) x values at once, then forms
 // the products.
-template <class E, int S, class W, bool SPLIT>
+template <class E, int S, class W>
 __device__ inline void stage_products(const PullRing<E, W>* ring, int b, const E* __restrict__ x,
                                       uint32_t e0, uint32_t count, E* stage, DeviceError* err,
-                                      uint32_t row, uint32_t hot, uint64_t keep) {
+                                      uint32_t row) {
   const unsigned lane = threadIdx.x & 31;
   constexpr int Q = kTileEntries / 32;
   const uint32_t* tg = ring->tgt[b] + (e0 & 3u);
   E xv[Q];
-  if constexpr (SPLIT) {
 #pragma unroll
-    for (int q = 0; q < Q; q++) {
-      const uint32_t k = lane + 32 * q;
-      if (k < count) xv[q] = load_x_split(x, tg[k], hot, keep);
-    }
-  } else {
-#pragma unroll
-    for (int q = 0; q < Q; q++) {
-      const uint32_t k = lane + 32 * q;
-      if (k < count) xv[q] = load_x(x, tg[k]);
-    }
+  for (int q = 0; q < Q; q++) {
+    const uint32_t k = lane + 32 * q;
+    if (k < count) xv[q] = load_x(x, tg[k]);
   }
 #pragma unroll
   for (int q = 0; q < Q; q++) {
@@ -287,13 +252,12 @@ __device__ inline void stage_products(const PullRing<E, W>* ring, int b, const E
 }
 
 // Walks the schedule, a warp per unit, the units of a warp strided by the
-// grid's warp count, through the warp's staging ring.  SPLIT: the CSC is in
-// locality order and A.hot splits the gathers (load_x_split).  The epilogue's
+// grid's warp count, through the warp's staging ring.  The epilogue's
 // per-row operands (`epi.pre(row)`) are requested as a unit starts, so they
 // arrive with its gathers.  `epi.row(row, present, value, pre)` is called
 // exactly once per row, by one lane.  A ring wait that runs out (about 2 s)
 // raises WC_DEVICE_TIMEOUT and ends the walk after the copies in flight.
-template <class E, int S, class W, class Epi, bool SPLIT = false, bool DEFER = false>
+template <class E, int S, class W, class Epi>
 __device__ inline void pull_units(const CsrView<W>& A, const E* __restrict__ x, Epi& epi,
                                   DeviceError* err, PullRing<E, W>* ring) {
   constexpr int R = PullRing<E, W>::R;
@@ -308,8 +272,6 @@ __device__ inline void pull_units(const CsrView<W>& A, const E* __restrict__ x, 
     for (int b = 0; b < R; b++) mbar_init(&ring->bar[b], 1);
   __syncwarp();
   const uint64_t stream = l2_evict_first_policy();
-  uint64_t keep = 0;
-  if constexpr (SPLIT) keep = l2_evict_last_policy();
   Unit ahead{0u, 0u, 0u, 0u};  // lane 0: the next unit to issue
   uint32_t pending = 0;        // buffers with a copy in flight (uniform)
   for (int b = 0; b < R; b++) {
@@ -347,7 +309,7 @@ __device__ inline void pull_units(const CsrView<W>& A, const E* __restrict__ x, 
         hi = soff[lane + 1];
         pre = epi.pre(r0 + lane);
       }
-      stage_products<E, S, W, SPLIT>(ring, b, x, e0, count, ring->stage, err, r0, A.hot, keep);
+      stage_products<E, S, W>(ring, b, x, e0, count, ring->stage, err, r0);
       __syncwarp();
       if (lane < rows) {
         E sum{};
@@ -372,7 +334,7 @@ __device__ inline void pull_units(const CsrView<W>& A, const E* __restrict__ x, 
       const uint32_t row = unit.a, e0 = unit.b, e1 = unit.d;
       const uint32_t slot = unit.c & 0x7fffffffu;
       const uint32_t count = e1 - e0;
-      stage_products<E, S, W, SPLIT>(ring, b, x, e0, count, ring->stage, err, row, A.hot, keep);
+      stage_products<E, S, W>(ring, b, x, e0, count, ring->stage, err, row);
       __syncwarp();
       Partial<E, ADD> mine{Acc<E, ADD>::of(E{}), false};
       constexpr uint32_t per = kTileEntries / 32;
@@ -382,33 +344,27 @@ __device__ inline void pull_units(const CsrView<W>& A, const E* __restrict__ x, 
         Partial<E, ADD> other = shfl_partial(mine, o);
         if ((lane & (2 * o - 1)) == 0) mine = join(mine, other);
       }
-      if constexpr (DEFER) {
-        // The piece's partial only: a later pass combines each long
-        // row's pieces in order (it starts after every piece is stored).
-        if (lane == 0) carry[slot] = mine;
-      } else {
-        const uint32_t row_lo = __ldg(A.off + row);
-        const uint32_t deg = __ldg(A.off + row + 1) - row_lo;
-        const uint32_t pieces = (deg + kPieceEntries - 1) / kPieceEntries;
-        const uint32_t first = slot - (e0 - row_lo) / kPieceEntries;
-        uint32_t arrived = 0;
+      const uint32_t row_lo = __ldg(A.off + row);
+      const uint32_t deg = __ldg(A.off + row + 1) - row_lo;
+      const uint32_t pieces = (deg + kPieceEntries - 1) / kPieceEntries;
+      const uint32_t first = slot - (e0 - row_lo) / kPieceEntries;
+      uint32_t arrived = 0;
+      if (lane == 0) {
+        carry[slot] = mine;
+        arrived = arrive_acq_rel(A.counters + first);
+      }
+      arrived = __shfl_sync(0xffffffffu, arrived, 0);
+      if (arrived == pieces - 1) {
+        __threadfence();
+        typename Epi::Pre pre{};
+        if (lane == 0) pre = epi.pre(row);
+        Partial<E, ADD> total = combine_pieces<E, ADD, 1>(carry, first, pieces, 0, lane);
         if (lane == 0) {
-          carry[slot] = mine;
-          arrived = arrive_acq_rel(A.counters + first);
-        }
-        arrived = __shfl_sync(0xffffffffu, arrived, 0);
-        if (arrived == pieces - 1) {
-          __threadfence();
-          typename Epi::Pre pre{};
-          if (lane == 0) pre = epi.pre(row);
-          Partial<E, ADD> total = combine_pieces<E, ADD, 1>(carry, first, pieces, 0, lane);
-          if (lane == 0) {
-            A.counters[first] = 0;
-            E v;
-            int32_t s = total.acc.value(&v);
-            if (s) raise(err, s, row);
-            epi.row(row, true, v, pre);
-          }
+          A.counters[first] = 0;
+          E v;
+          int32_t s = total.acc.value(&v);
+          if (s) raise(err, s, row);
+          epi.row(row, true, v, pre);
         }
       }
     }
@@ -457,7 +413,7 @@ template <class E, int S> struct WriteEpi {
     if (w.accumulate >= 0 && p.selected) p.old = y[row];
     return p;
   }
-  __device__ void row(uint32_t row, bool present, E t, const Pre& p) {
+  __device__ void row(uint32_t row, bool present, E t, const Pre& p, void* = nullptr) {
     const E identity = Identity<E>::of(semiring_add(S));
     if (!p.selected) {
       if (w.replace) y[row] = identity;

@@ -243,20 +243,53 @@ struct Schedule {
   uint32_t tiles = 0;
 };
 
+// A CSR orientation's entries laid out for a warp's lanes to fold the rows
+// they gather for (lanes.cu builds it, lanes.cuh walks it): rows of at most
+// kPieceEntries entries sorted by length and cut into slices, g = 1 or 8 lanes
+// a row, entry k of the row whose lanes start at l in its step k / g, at
+// base + 32 (k / g) + l + k % g; the longer
+// rows' pieces laid out likewise, eight consecutive entries a lane.
+// Targets among the `hot_count` most gathered nodes hold kHotTarget | slot.
+constexpr uint32_t kHotTarget = 0x80000000u;
+struct LaneUnit {
+  // slice: first of `rows`, steps, base / 32, log2 g | rows << 8 | the
+  // entries that every lane has (at least) << 16;
+  // pieces [f, f + np) of long row a: b = f << 8 | np, base / 32 of the
+  // first, d = 1 << 31 | the row's first carry slot.
+  uint32_t a, b, c, d;
+};
+struct LaneCsr {
+  DevBuf units;              // LaneUnit[count]
+  DevBuf rows, lengths;      // u32 / u16: row ids sorted by length, longest first; their entries
+  DevBuf targets, weights, iweights;
+  DevBuf hot;                // u32[hot_count]: the hot nodes, most gathered first
+  uint32_t count = 0;
+  uint32_t filled = 0, shorts = 0;  // of `rows`: those with entries, then to here the empty ones
+  uint32_t hot_count = 0;
+  uint32_t run = 1;     // pieces of a long row a unit takes at most
+  uint64_t places = 0;  // entries' places, padding among them (its targets 0)
+  uint64_t bytes() const {
+    return units.bytes + rows.bytes + lengths.bytes + targets.bytes + weights.bytes +
+           iweights.bytes + hot.bytes;
+  }
+};
+
 // One CSR orientation on the device: u32 offsets and targets, f64 weights
 // (absent when unweighted) and, when every weight is an integer in int32
 // range, an int32 copy for the integer semirings.
 struct DevCsr {
   DevBuf offsets, targets, weights, iweights;
   Schedule schedule;
+  LaneCsr lanes;  // the version's two orientations only
   uint32_t max_degree = 0;
 };
 
-// The reverse CSR in locality order (locality.cu): nodes renumbered by
-// out-degree, largest first; perm maps a dense id to its new number and
-// order a new number back to the dense id.
+// The reverse CSR in row order (locality.cu): nodes renumbered by the length
+// of their reverse rows, longest first; perm maps a dense id to its new
+// number and order a new number back to the dense id.
 struct Locality {
   DevBuf perm, order;  // u32[n] each
+  DevBuf lane_targets, lane_hot;  // rev.lanes' targets and hot nodes, renumbered
   DevCsr csc;
 };
 

@@ -2,6 +2,7 @@
 // Y = A ⊗ X (SpMM), instantiated once per element type in spmv_<dtype>.cu.
 #pragma once
 
+#include "lanes.cuh"
 #include "pull.cuh"
 #include "pull_multi.cuh"
 #include "product.h"
@@ -14,6 +15,15 @@ __global__ void __launch_bounds__(kPullThreads, 3)
   extern __shared__ __align__(16) unsigned char smem[];
   PullRing<E, W>* ring = reinterpret_cast<PullRing<E, W>*>(smem) + (threadIdx.x >> 5);
   pull_units<E, S, W>(A, x, epi, err, ring);
+}
+
+template <class E, int S, class W>
+__global__ void __launch_bounds__(kLaneThreads, 1)
+    spmv_lane_kernel(LaneView<W> A, const E* __restrict__ x, WriteEpi<E, S> epi, DeviceError* err) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  E* hot = reinterpret_cast<E*>(smem);
+  lane_fill_hot<E, W>(A, x, hot);
+  lane_units<E, S, W>(A, x, hot, epi, err);
 }
 
 // SpMM, width > 1: the multi-column pull (pull_multi.cuh) over a block of
@@ -58,7 +68,17 @@ template <class E, int S, class W>
 wc_status launch_one(const PullLaunch& L, const void* x, void* y) {
   CsrView<W> A{L.off, L.tgt, static_cast<const W*>(L.weights), L.units, L.unit_count,
                L.counters, L.carry};
-  if (L.width == 1) {
+  if (L.width == 1 && L.lanes) {
+    WriteEpi<E, S> epi{L.write, static_cast<E*>(y), L.err};
+    static const cudaError_t attr = cudaFuncSetAttribute(
+        spmv_lane_kernel<E, S, W>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        (int)(kHotSlots * sizeof(E)));
+    if (attr != cudaSuccess) return cuda_status(attr, L.detail, "product kernel attributes");
+    const LaneView<W> V = lane_view<W>(L);
+    note_launch(), spmv_lane_kernel<E, S, W><<<lane_grid(L), kLaneThreads,
+                                               V.hot_count * sizeof(E), L.stream>>>(
+        V, static_cast<const E*>(x), epi, L.err);
+  } else if (L.width == 1) {
     WriteEpi<E, S> epi{L.write, static_cast<E*>(y), L.err};
     constexpr size_t smem = pull_smem_bytes<E, W>();
     static const cudaError_t attr = cudaFuncSetAttribute(

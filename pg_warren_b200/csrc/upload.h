@@ -26,6 +26,12 @@ wc_status finish_version(wc_version* v, wc_error_detail* detail);
 // The row-split schedule of one orientation from its host offsets.
 wc_status put_schedule(wc_version* v, DevCsr& d, const std::vector<uint64_t>& off,
                        wc_error_detail* detail);
+// The lane-major copy of `d` (v->fwd or v->rev), after its schedule: `off`
+// are its host offsets, `other` the other orientation (whose row lengths say
+// how often each node is gathered) and `other_off` its host offsets.
+wc_status device_lanes(wc_version* v, DevCsr& d, const std::vector<uint64_t>& off,
+                       const DevCsr& other, const std::vector<uint64_t>& other_off,
+                       wc_error_detail* detail);
 // The reverse CSR in locality order (v->loc), after the weights' facts.
 wc_status device_locality(wc_version* v, wc_error_detail* detail);
 // Vectors between dense ids and the locality numbering, on `st`:

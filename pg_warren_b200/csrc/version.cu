@@ -158,6 +158,8 @@ wc_status finish_version(wc_version* v, wc_error_detail* detail) {
   WC_TRY(device_symmetric(v, detail));
   WC_TRY(put_schedule(v, v->fwd, v->host_offsets, detail));
   WC_TRY(put_schedule(v, v->rev, v->host_rev_offsets, detail));
+  WC_TRY(device_lanes(v, v->fwd, v->host_offsets, v->rev, v->host_rev_offsets, detail));
+  WC_TRY(device_lanes(v, v->rev, v->host_rev_offsets, v->fwd, v->host_offsets, detail));
   WC_TRY(device_locality(v, detail));
   WC_TRY(v->error.alloc(v->budget, sizeof(DeviceError), detail));
   WC_CUDA(cudaMemset(v->error.ptr, 0, sizeof(DeviceError)), detail);
@@ -312,8 +314,9 @@ wc_status wc_version_info_get(const wc_version* v, wc_version_info* info) {
   for (const DevCsr* d : {&v->fwd, &v->rev, &v->loc.csc})
     bytes += d->offsets.bytes + d->targets.bytes + d->weights.bytes + d->iweights.bytes +
              d->schedule.units.bytes + d->schedule.counters.bytes + d->schedule.carry.bytes +
-             d->schedule.long_list.bytes + d->schedule.row_masks.bytes;
-  bytes += v->loc.perm.bytes + v->loc.order.bytes;
+             d->schedule.long_list.bytes + d->schedule.row_masks.bytes + d->lanes.bytes();
+  bytes += v->loc.perm.bytes + v->loc.order.bytes + v->loc.lane_targets.bytes +
+           v->loc.lane_hot.bytes;
   info->device_bytes = bytes;
   uint64_t pooled = 0;
   for (const auto& kv : v->pool) pooled += kv.second.bytes;
