@@ -127,9 +127,8 @@ __global__ void __launch_bounds__(256) adj_rows_kernel(CsrView<W> A, AdjState s,
   pull_multi<double, WC_PLUS_TIMES, W, P>(A, s.lam[cur], epi, s.err, carry);
 }
 
-// The same iteration and final pass over pull32_units (cp.async gathers
-// into a per-warp ring, small blocks, as many warps an SM as the registers
-// allow): a lane is a loss; a loss that has stopped gathers nothing and
+// The same iteration and final pass over pull32_units (small blocks, as many
+// warps an SM as the registers allow): a lane is a loss; a loss that has stopped gathers nothing and
 // keeps its λ.
 struct AdjEpi32 {
   struct Row {
@@ -146,44 +145,50 @@ struct AdjEpi32 {
   __device__ Row shfl(const Row& r, uint32_t src) const {
     return Row{__shfl_sync(0xffffffffu, r.out, src)};
   }
-  __device__ void emit(uint32_t i, const Partial<double, WC_OP_PLUS>& acc, const Row& r) {
+  // λ's column and, but in the final pass, the loss indicator's.
+  struct Old {
+    double lam, c;
+  };
+  __device__ Old old(uint32_t i) const {
+    if (final_pass) return Old{};
+    const size_t at = (size_t)i * 32 + (threadIdx.x & 31);
+    return Old{s->lam[cur][at], s->C[at]};
+  }
+  __device__ void emit(uint32_t i, bool present, double z, const Old& was, const Row& r) {
     const AdjState& st = *s;
     const unsigned c = threadIdx.x & 31;
     const size_t at = (size_t)i * 32 + c;
-    double z = 0.0;
-    if (acc.present) acc.acc.value(&z);
     const double o = r.out;
-    const double si = (acc.present && o > 0.0) ? z / o : 0.0;
+    const double si = (present && o > 0.0) ? z / o : 0.0;
     if (final_pass) {
       st.S[at] = si;
       return;
     }
-    const double old = st.lam[cur][at];
     if (!((run_bits >> c) & 1)) {
-      st.lam[cur ^ 1][at] = old;
-      total += old;
+      st.lam[cur ^ 1][at] = was.lam;
+      total += was.lam;
       return;
     }
-    const double next = st.damping * (si + (o > 0.0 ? 0.0 : pi)) + st.C[at];
-    delta += fabs(next - old);
+    const double next = st.damping * (si + (o > 0.0 ? 0.0 : pi)) + was.c;
+    delta += fabs(next - was.lam);
     total += next;
     st.lam[cur ^ 1][at] = next;
   }
 };
 
 template <class W>
-__global__ void __launch_bounds__(kPull32Warps * 32, 6)
+__global__ void __launch_bounds__(kPull32Warps * 32, 5)
     adj_iter32_kernel(CsrView<W> A, AdjState s, uint32_t it, Partial<double, WC_OP_PLUS>* carry,
                       uint32_t max_iter) {
   const uint32_t run = *(volatile uint32_t*)s.running;
   if (!run) return;
-  extern __shared__ __align__(16) double adj_smem[];
+  extern __shared__ __align__(16) unsigned char adj_smem[];
   const unsigned c = threadIdx.x & 31;
   AdjEpi32 epi{&s, (int)(it & 1), run, s.pi[c]};
   epi.final_pass = false;
   epi.active = (run >> c) & 1;
   pull32_units<W>(A, s.lam[it & 1], epi, s.err, carry,
-                  adj_smem + (threadIdx.x >> 5) * kPull32WarpDoubles);
+                  reinterpret_cast<Pull32Warp<W>*>(adj_smem)[threadIdx.x >> 5]);
   double delta = epi.delta, total = epi.total;
   if (reduce_columns<32>(delta, total, s.partials, s.counter)) {
     const uint32_t q = threadIdx.x;
@@ -197,16 +202,16 @@ __global__ void __launch_bounds__(kPull32Warps * 32, 6)
 }
 
 template <class W>
-__global__ void __launch_bounds__(kPull32Warps * 32, 6)
+__global__ void __launch_bounds__(kPull32Warps * 32, 5)
     adj_rows32_kernel(CsrView<W> A, AdjState s, Partial<double, WC_OP_PLUS>* carry) {
-  extern __shared__ __align__(16) double adj_smem[];
+  extern __shared__ __align__(16) unsigned char adj_smem[];
   const int cur = *s.executed & 1;
   const unsigned c = threadIdx.x & 31;
   AdjEpi32 epi{&s, cur, 0, 0.0};
   epi.final_pass = true;
   epi.active = c < s.k;
   pull32_units<W>(A, s.lam[cur], epi, s.err, carry,
-                  adj_smem + (threadIdx.x >> 5) * kPull32WarpDoubles);
+                  reinterpret_cast<Pull32Warp<W>*>(adj_smem)[threadIdx.x >> 5]);
 }
 
 // grad[c][e] = d · x_i / out_i · (λ_j − S_i) for e = (i → j), a warp per
@@ -262,11 +267,11 @@ __global__ void adj_targets_kernel(const uint64_t* targets, const uint64_t* offs
     atomicAdd(C + (size_t)targets[q] * kAdjP + c, 1.0);
 }
 
-// The iterations' blocks: kPull32Warps warps, at most one warp a unit; six
-// an SM (the kernels are held to 80 registers for it: 6% faster on R-MAT 22
-// than five at 96, where the batched PPR's pull is slower at 80).
+// The iterations' blocks: kPull32Warps warps, at most one warp a unit; five
+// an SM (six at 80 registers leave eight gathers in flight: level, 29.5 ms
+// over R-MAT 18's 32 losses).
 static uint32_t adjoint_grid32(const DevCsr& fwd) {
-  return std::max<uint32_t>(1, std::min<uint32_t>(max_blocks(6),
+  return std::max<uint32_t>(1, std::min<uint32_t>(max_blocks(5),
                                                   (fwd.schedule.count + kPull32Warps - 1) /
                                                       kPull32Warps));
 }
@@ -280,14 +285,14 @@ static wc_status adjoint_pass(Ctx& ctx, AdjState& s, const DevCsr& fwd, const vo
                fwd.schedule.counters.as<uint32_t>(), nullptr};
   const uint32_t grid32 = adjoint_grid32(fwd);
   WC_CUDA(cudaFuncSetAttribute(adj_iter32_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)kPull32Smem), ctx.detail);
+                               (int)pull32_smem<W>()), ctx.detail);
   WC_CUDA(cudaFuncSetAttribute(adj_rows32_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)kPull32Smem), ctx.detail);
+                               (int)pull32_smem<W>()), ctx.detail);
   note_launch(), adj_init_kernel<kAdjP><<<grid, 256, 0, ctx.stream>>>(s);
   for (uint32_t it = 0; it < max_iter; it++)
-    note_launch(), adj_iter32_kernel<W><<<grid32, kPull32Warps * 32, kPull32Smem, ctx.stream>>>(
+    note_launch(), adj_iter32_kernel<W><<<grid32, kPull32Warps * 32, pull32_smem<W>(), ctx.stream>>>(
         A, s, it, carry, max_iter);
-  note_launch(), adj_rows32_kernel<W><<<grid32, kPull32Warps * 32, kPull32Smem, ctx.stream>>>(
+  note_launch(), adj_rows32_kernel<W><<<grid32, kPull32Warps * 32, pull32_smem<W>(), ctx.stream>>>(
       A, s, carry);
   note_launch(), adj_scatter_kernel<kAdjP><<<max_blocks(8), 256, 0, ctx.stream>>>(
       fwd.offsets.as<uint32_t>(), fwd.targets.as<uint32_t>(), fwd.schedule.units.as<Unit>(),

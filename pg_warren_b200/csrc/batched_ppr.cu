@@ -78,11 +78,16 @@ struct PprStream {
   DeviceError* err;
 };
 
+__device__ __noinline__ void ppr_check_spread(double x, double out, DeviceError* err, uint32_t i) {
+  double m;
+  const int32_t s = sql_float<F_DIV>(x, out, &m);
+  if (s) raise(err, s, i);
+}
+
 __device__ inline double ppr_spread(double x, double out, double* msg, DeviceError* err, uint32_t i) {
   if (sql_cmp_f(out, 0.0) > 0) {
-    double m;
-    int32_t s = sql_float<F_DIV>(x, out, &m);
-    if (s) raise(err, s, i);
+    const double m = x / out;
+    if ((m == 0.0 && x != 0.0) || !isfinite(m)) ppr_check_spread(x, out, err, i);
     *msg = m;
     return 0.0;
   }
@@ -235,7 +240,20 @@ __global__ void __launch_bounds__(256) ppr_iter_kernel(CsrView<W> A, PprStream s
 
 // ------------------------------------------------------ the 32-slot pull
 // With 32 slots the iteration is pull32_units (pull32.cuh) with the rank
-// update as its epilogue; it is bound by instruction issue, not bandwidth.
+// update as its epilogue.
+
+// A node's next rank by the reference's checked operations.
+__device__ __noinline__ double ppr_checked(double damping, double teleport, DeviceError* err,
+                                           uint32_t i, double y, double p, double dangling_in) {
+  double dp, flowed, a, b, next = 0.0;
+  int32_t e = sql_float<F_MUL>(dangling_in, p, &dp);
+  if (!e) e = sql_float<F_ADD>(y, dp, &flowed);
+  if (!e) e = sql_float<F_MUL>(damping, flowed, &a);
+  if (!e) e = sql_float<F_MUL>(teleport, p, &b);
+  if (!e) e = sql_float<F_ADD>(a, b, &next);
+  if (e) raise(err, e, i);
+  return next;
+}
 
 // The rank update of row i for this lane's slot (pagerank/mod.rs:201-282).
 struct PprEpi32 {
@@ -248,7 +266,7 @@ struct PprEpi32 {
   const double* XO;
   double* XN;
   double* MN;
-  double dangling_in, share;
+  double dangling_in, share, damping;
   double delta = 0.0, dangling_out = 0.0;
   bool active;
   __device__ Row row(uint32_t i) const {
@@ -258,27 +276,30 @@ struct PprEpi32 {
     return Row{__shfl_sync(0xffffffffu, r.mem, src), __shfl_sync(0xffffffffu, r.out, src),
                __shfl_sync(0xffffffffu, r.dead, src) != 0};
   }
-  __device__ void emit(uint32_t i, const Partial<double, WC_OP_PLUS>& acc, const Row& r) {
+  struct Old {
+    double x;
+  };
+  __device__ Old old(uint32_t i) const {
+    return Old{active ? XO[(size_t)i * 32 + (threadIdx.x & 31)] : 0.0};
+  }
+  // A node outside the slot's set has no personalisation, so its rank is
+  // damping · y.  Every failing operation leaves an infinity, a NaN or a zero
+  // product, so only a row that shows one, or is in a set, goes through the
+  // checked operations.
+  __device__ void emit(uint32_t i, bool present, double y, const Old& was, const Row& r) {
     if (!active) return;
     const unsigned lane = threadIdx.x & 31;
-    const PprStream& st = *s;
-    const double old = XO[(size_t)i * 32 + lane];
-    double y = 0.0;
-    if (acc.present) acc.acc.value(&y);
-    double next = 0.0;
-    if (!r.dead) {
-      const double p = ((r.mem >> lane) & 1) ? share : 0.0;
-      double dp, flowed, a, b;
-      int32_t e = sql_float<F_MUL>(dangling_in, p, &dp);
-      if (!e) e = sql_float<F_ADD>(y, dp, &flowed);
-      if (!e) e = sql_float<F_MUL>(st.damping, flowed, &a);
-      if (!e) e = sql_float<F_MUL>(st.teleport, p, &b);
-      if (!e) e = sql_float<F_ADD>(a, b, &next);
-      if (e) raise(st.err, e, i);
-    }
-    delta += fabs(next - old);
-    XN[(size_t)i * 32 + lane] = next;
-    dangling_out += ppr_spread(next, r.out, &MN[(size_t)i * 32 + lane], st.err, i);
+    if (!present) y = 0.0;
+    double next = damping * y;
+    if (r.dead)
+      next = 0.0;
+    else if (((r.mem >> lane) & 1) || !isfinite(next) || (next == 0.0 && y != 0.0))
+      next = ppr_checked(damping, s->teleport, s->err, i, y, ((r.mem >> lane) & 1) ? share : 0.0,
+                         dangling_in);
+    delta += fabs(next - was.x);
+    const size_t at = (size_t)i * 32 + lane;
+    XN[at] = next;
+    dangling_out += ppr_spread(next, r.out, &MN[at], s->err, i);
   }
 };
 
@@ -294,14 +315,15 @@ __global__ void __launch_bounds__(kPull32Warps * 32, 5)
     }
     return;
   }
-  extern __shared__ __align__(16) double ppr_smem[];
+  extern __shared__ __align__(16) unsigned char ppr_smem[];
   const uint32_t g = *(volatile uint32_t*)&ctl->g;
   const int cur = g & 1;
   const unsigned lane = threadIdx.x & 31;
-  PprEpi32 epi{&s, s.x[cur], s.x[cur ^ 1], s.msg[cur ^ 1], ctl->dangling[lane], ctl->share[lane]};
+  PprEpi32 epi{&s, s.x[cur], s.x[cur ^ 1], s.msg[cur ^ 1], ctl->dangling[lane], ctl->share[lane],
+               s.damping};
   epi.active = (run >> lane) & 1;
   pull32_units<W>(A, s.msg[cur], epi, s.err, carry,
-                  ppr_smem + (threadIdx.x >> 5) * kPull32WarpDoubles);
+                  reinterpret_cast<Pull32Warp<W>*>(ppr_smem)[threadIdx.x >> 5]);
   double delta = epi.delta, dangling_out = epi.dangling_out;
   if (reduce_columns<32>(delta, dangling_out, s.partials, &ctl->counter))
     ppr_control<32>(s, run, g, delta, dangling_out);
@@ -388,12 +410,13 @@ static void ppr_queue_iteration(Ctx& ctx, const PprStream& s, uint32_t grid, boo
                                 Partial<double, WC_OP_PLUS>* carry) {
   wc_version* v = ctx.v;
   if constexpr (P == 32) {
-    constexpr size_t smem32 = kPull32Smem;
     if (weighted)
-      note_launch(), ppr_iter32_kernel<double><<<grid, kPull32Warps * 32, smem32, ctx.stream>>>(
+      note_launch(), ppr_iter32_kernel<double><<<grid, kPull32Warps * 32, pull32_smem<double>(),
+                                                 ctx.stream>>>(
           view_of<double>(v->loc.csc, v->loc.csc.weights.ptr), s, carry);
     else
-      note_launch(), ppr_iter32_kernel<void><<<grid, kPull32Warps * 32, smem32, ctx.stream>>>(
+      note_launch(), ppr_iter32_kernel<void><<<grid, kPull32Warps * 32, pull32_smem<void>(),
+                                               ctx.stream>>>(
           view_of<void>(v->loc.csc, nullptr), s, carry);
   } else {
     if (weighted)
@@ -459,11 +482,12 @@ wc_status ppr_stream(Ctx& ctx, const PageRankRun& base, const uint64_t* nodes,
   const bool weighted = base.opts.weighted != 0 && v->weighted;
   auto* carry = cb->as<Partial<double, WC_OP_PLUS>>();
   if constexpr (P == 32) {
-    constexpr int smem32 = (int)kPull32Smem;
     WC_CUDA(cudaFuncSetAttribute(ppr_iter32_kernel<double>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, smem32), ctx.detail);
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)pull32_smem<double>()), ctx.detail);
     WC_CUDA(cudaFuncSetAttribute(ppr_iter32_kernel<void>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, smem32), ctx.detail);
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)pull32_smem<void>()), ctx.detail);
   }
   // Greedy hand-out over P slots: no slot runs longer than the mean load
   // plus one set, so this many global iterations always finish every set.
