@@ -46,34 +46,6 @@ struct Rows {  // the rows read in one direction: one CSR, or two for Both
   }
 };
 
-// Appends v to the next frontier and marks it in the next frontier's
-// bitmap: one atomic per warp for the lanes that admit a node this round.
-__device__ inline void admit(uint32_t v, bool take, uint32_t* next, uint32_t* fnext,
-                             LevelState* c, const Rows& adj, const Rows& radj) {
-  const unsigned mask = __ballot_sync(0xffffffffu, take);
-  if (!mask) return;
-  const unsigned lane = threadIdx.x & 31;
-  const int leader = __ffs(mask) - 1;
-  uint32_t base = 0;
-  if ((int)lane == leader) base = atomicAdd(&c->next_count, (uint32_t)__popc(mask));
-  base = __shfl_sync(0xffffffffu, base, leader);
-  unsigned long long d = 0, rd = 0;
-  if (take) {
-    next[base + __popc(mask & ((1u << lane) - 1))] = v;
-    atomicOr(fnext + (v >> 5), 1u << (v & 31));
-    d = adj.degree(v);
-    rd = radj.degree(v);
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    d += __shfl_down_sync(0xffffffffu, d, o);
-    rd += __shfl_down_sync(0xffffffffu, rd, o);
-  }
-  if (lane == 0) {
-    atomicAdd(&c->next_deg, d);
-    atomicAdd(&c->next_rdeg, rd);
-  }
-}
-
 // What every kernel of a level is given.
 struct LevelArgs {
   Rows adj, radj;
@@ -96,10 +68,12 @@ struct LevelArgs {
 // Levels queued per round trip to the host.
 constexpr uint32_t kChunkLevels = 16;
 
-// Rows longer than this are pushed by a block each (push_big_kernel): one
-// warp per row would leave a hub's row to a single warp.  Rows longer than
+// Rows longer than this are pushed by a block each (push_big_kernel): a warp
+// takes 128 entries at a time, each a chain of dependent loads and atomics
+// (about 2 µs), so a hub's row left to a single warp is what the level waits
+// for: at 2,048 a level of R-MAT 16 took 100 µs.  Rows longer than
 // kHugeRow are pushed by the whole grid, one after another.
-constexpr uint32_t kBigRow = 2048;
+constexpr uint32_t kBigRow = 512;
 constexpr uint32_t kHugeRow = 32768;
 
 // The long-row list's entries: at most one per kBigRow entries of the rows
@@ -108,14 +82,69 @@ inline uint32_t big_entries(uint64_t m, int dir) {
   return (uint32_t)((m / kBigRow + 2) * (dir == WC_BOTH ? 2 : 1));
 }
 
-// One entry of a push: target v offered by frontier node u.
-__device__ inline bool offer(const LevelArgs& a, uint32_t u, uint32_t v) {
-  const bool allowed = !a.filter || ((a.filter[v >> 6] >> (v & 63)) & 1);
-  if (!allowed) return false;
-  const uint32_t d = a.depth[v];
-  if (d != WC_UNREACHED && d != a.depth_next) return false;
-  atomicMin(a.via + v, (unsigned long long)u);
-  return d == WC_UNREACHED && atomicCAS(a.depth + v, WC_UNREACHED, a.depth_next) == WC_UNREACHED;
+// Appends the nodes v[q] that are taken (up to N a lane) to the next frontier
+// and marks them in its bitmap: one atomic a warp for the queue, so N rounds'
+// chains of dependent atomics pass as one.
+template <int N>
+__device__ inline void admit(const uint32_t (&v)[N], const bool (&take)[N], const LevelArgs& a) {
+  uint32_t mine = 0;
+#pragma unroll
+  for (int q = 0; q < N; q++) mine += take[q];
+  if (!__any_sync(0xffffffffu, mine != 0)) return;
+  const unsigned lane = threadIdx.x & 31;
+  uint32_t at = mine;  // the lanes' counts, summed up to and including this one
+#pragma unroll
+  for (unsigned o = 1; o < 32; o <<= 1) {
+    const uint32_t below = __shfl_up_sync(0xffffffffu, at, o);
+    if (lane >= o) at += below;
+  }
+  uint32_t base = 0;
+  if (lane == 31) base = atomicAdd(&a.st->next_count, at);
+  at += __shfl_sync(0xffffffffu, base, 31) - mine;
+  unsigned long long d = 0, rd = 0;
+#pragma unroll
+  for (int q = 0; q < N; q++)
+    if (take[q]) {
+      a.next[at++] = v[q];
+      atomicOr(a.fnext + (v[q] >> 5), 1u << (v[q] & 31));
+      d += a.adj.degree(v[q]);
+      rd += a.radj.degree(v[q]);
+    }
+  for (int o = 16; o > 0; o >>= 1) {
+    d += __shfl_down_sync(0xffffffffu, d, o);
+    rd += __shfl_down_sync(0xffffffffu, rd, o);
+  }
+  if (lane == 0) {
+    atomicAdd(&a.st->next_deg, d);
+    atomicAdd(&a.st->next_rdeg, rd);
+  }
+}
+
+// Entries e, e + stride, ... (kPushEntries of them, below `hi`) of frontier
+// node u's row offered to their targets.
+constexpr int kPushEntries = 4;
+__device__ inline void offer_entries(const LevelArgs& a, const uint32_t* tgt, uint32_t u,
+                                     uint64_t e, uint64_t stride, uint32_t hi) {
+  uint32_t v[kPushEntries], d[kPushEntries];
+  bool take[kPushEntries], open[kPushEntries];
+#pragma unroll
+  for (int q = 0; q < kPushEntries; q++) {
+    open[q] = e + q * stride < hi;
+    v[q] = open[q] ? __ldg(tgt + e + q * stride) : 0u;
+  }
+#pragma unroll
+  for (int q = 0; q < kPushEntries; q++) {
+    if (open[q] && a.filter) open[q] = (a.filter[v[q] >> 6] >> (v[q] & 63)) & 1;
+    d[q] = open[q] ? a.depth[v[q]] : 0u;
+  }
+#pragma unroll
+  for (int q = 0; q < kPushEntries; q++) {
+    open[q] = open[q] && (d[q] == WC_UNREACHED || d[q] == a.depth_next);
+    if (open[q]) atomicMin(a.via + v[q], (unsigned long long)u);
+    take[q] = open[q] && d[q] == WC_UNREACHED &&
+              atomicCAS(a.depth + v[q], WC_UNREACHED, a.depth_next) == WC_UNREACHED;
+  }
+  admit(v, take, a);
 }
 
 // Push: a warp per frontier node, lanes over its row entries; rows longer
@@ -139,16 +168,8 @@ __device__ inline void push_level(const LevelArgs& a) {
       const uint32_t* tgt = part == 0 ? a.adj.tgt0 : a.adj.tgt1;
       if (!off) break;
       const uint32_t lo = __ldg(off + u), hi = __ldg(off + u + 1);
-      for (uint32_t e0 = lo; e0 < hi; e0 += 32) {
-        const uint32_t e = e0 + lane;
-        bool take = false;
-        uint32_t v = 0;
-        if (e < hi) {
-          v = __ldg(tgt + e);
-          take = offer(a, u, v);
-        }
-        admit(v, take, a.next, a.fnext, a.st, a.adj, a.radj);
-      }
+      for (uint64_t e0 = lo; e0 < hi; e0 += 32 * kPushEntries)
+        offer_entries(a, tgt, u, e0 + lane, 32, hi);
     }
   }
 }
@@ -178,16 +199,9 @@ __device__ inline void push_row_part(const LevelArgs& a, uint32_t u, uint32_t fi
     const uint32_t* tgt = part == 0 ? a.adj.tgt0 : a.adj.tgt1;
     if (!off) break;
     const uint32_t lo = __ldg(off + u), hi = __ldg(off + u + 1);
-    for (uint32_t e0 = lo + 32 * first_warp; e0 < hi; e0 += 32 * warp_stride) {
-      const uint32_t e = e0 + lane;
-      bool take = false;
-      uint32_t v = 0;
-      if (e < hi) {
-        v = __ldg(tgt + e);
-        take = offer(a, u, v);
-      }
-      admit(v, take, a.next, a.fnext, a.st, a.adj, a.radj);
-    }
+    const uint64_t stride = 32 * (uint64_t)warp_stride;
+    for (uint64_t e0 = lo + 32 * (uint64_t)first_warp; e0 < hi; e0 += stride * kPushEntries)
+      offer_entries(a, tgt, u, e0 + lane, stride, hi);
   }
 }
 
@@ -225,6 +239,48 @@ __global__ void __launch_bounds__(256) push_big_kernel(LevelArgs a, SwitchArgs s
   }
 }
 
+// The first frontier node in [lo, hi) of each lane's row (its position, hi
+// when there is none): the lane's own first kPullEntries entries, loaded at
+// once, then what is left of each lane's row by the whole warp, 32 entries at
+// a time (a hub's row left to one lane is what a level would wait for).
+constexpr int kPullEntries = 8;
+__device__ inline uint32_t first_in_frontier(const uint32_t* tgt, const uint32_t* fbits,
+                                             uint32_t lo, uint32_t hi, uint32_t& node) {
+  const unsigned lane = threadIdx.x & 31;
+  uint32_t v[kPullEntries];
+  uint32_t pos = hi;
+#pragma unroll
+  for (int q = 0; q < kPullEntries; q++) v[q] = lo + q < hi ? __ldg(tgt + lo + q) : 0u;
+#pragma unroll
+  for (int q = kPullEntries - 1; q >= 0; q--)
+    if (lo + q < hi && bit_at(fbits, v[q])) {
+      pos = lo + q;
+      node = v[q];
+    }
+  uint32_t rest = __ballot_sync(0xffffffffu, pos == hi && hi - lo > kPullEntries);
+  while (rest) {
+    const int src = __ffs(rest) - 1;
+    rest &= rest - 1;
+    const uint32_t end = __shfl_sync(0xffffffffu, hi, src);
+    uint32_t e0 = __shfl_sync(0xffffffffu, lo, src) + kPullEntries;
+    for (; e0 < end; e0 += 32) {
+      const uint32_t e = e0 + lane;
+      const uint32_t t = e < end ? __ldg(tgt + e) : 0u;
+      const uint32_t hit = __ballot_sync(0xffffffffu, e < end && bit_at(fbits, t));
+      if (hit) {
+        const int first = __ffs(hit) - 1;
+        const uint32_t at = __shfl_sync(0xffffffffu, t, first);
+        if ((int)lane == src) {
+          pos = e0 + first;
+          node = at;
+        }
+        break;
+      }
+    }
+  }
+  return pos;
+}
+
 // Pull: a thread per unvisited node, scanning its rows of `radj` (the
 // opposite direction), in order, to the first frontier node.  For Both the
 // smallest first hit of the two rows is `via` (what a push finds), while
@@ -237,32 +293,31 @@ __device__ inline void pull_level(const LevelArgs& a) {
   const uint32_t rounds = (n + stride - 1) / stride;
   for (uint32_t r = 0; r < rounds; r++) {
     const uint32_t v = r * stride + blockIdx.x * blockDim.x + threadIdx.x;
-    bool take = false;
-    if (v < n && a.depth[v] == WC_UNREACHED && (!a.filter || ((a.filter[v >> 6] >> (v & 63)) & 1))) {
-      uint64_t best = WC_NO_VIA;
-      bool counting = true;
+    const bool open = v < n && a.depth[v] == WC_UNREACHED &&
+                      (!a.filter || ((a.filter[v >> 6] >> (v & 63)) & 1));
+    uint64_t best = WC_NO_VIA;
+    bool counting = open;
+    if (__any_sync(0xffffffffu, open))
       for (int part = 0; part < 2; part++) {
         const uint32_t* off = part == 0 ? a.radj.off0 : a.radj.off1;
         const uint32_t* tgt = part == 0 ? a.radj.tgt0 : a.radj.tgt1;
         if (!off) break;
-        const uint32_t lo = __ldg(off + v), hi = __ldg(off + v + 1);
-        for (uint32_t e = lo; e < hi; e++) {
-          const uint32_t u = __ldg(tgt + e);
-          if (counting) scanned++;
-          if (bit_at(a.fbits, u)) {
-            if (u < best) best = u;
-            counting = false;
-            break;
-          }
+        const uint32_t lo = open ? __ldg(off + v) : 0u, hi = open ? __ldg(off + v + 1) : 0u;
+        uint32_t u = 0;
+        const uint32_t pos = first_in_frontier(tgt, a.fbits, lo, hi, u);
+        if (counting) scanned += pos < hi ? pos - lo + 1 : hi - lo;
+        if (pos < hi) {
+          if (u < best) best = u;
+          counting = false;
         }
       }
-      if (best != WC_NO_VIA) {
-        a.depth[v] = a.depth_next;
-        a.via[v] = best;
-        take = true;
-      }
+    const bool take[1] = {best != WC_NO_VIA};
+    if (take[0]) {
+      a.depth[v] = a.depth_next;
+      a.via[v] = best;
     }
-    admit(v, take, a.next, a.fnext, a.st, a.adj, a.radj);
+    const uint32_t node[1] = {v};
+    admit(node, take, a);
   }
   for (int o = 16; o > 0; o >>= 1) scanned += __shfl_down_sync(0xffffffffu, scanned, o);
   if ((threadIdx.x & 31) == 0 && scanned) atomicAdd(&a.st->edges, scanned);
