@@ -2,10 +2,12 @@
 // Y = A ⊗ X (SpMM), instantiated once per element type in spmv_<dtype>.cu.
 #pragma once
 
+#include <type_traits>
+
 #include "lanes.cuh"
 #include "pull.cuh"
-#include "pull_multi.cuh"
 #include "product.h"
+#include "spmm_rows.cuh"
 
 namespace wc {
 
@@ -26,42 +28,72 @@ __global__ void __launch_bounds__(kLaneThreads, 1)
   lane_units<E, S, W>(A, x, hot, epi, err);
 }
 
-// SpMM, width > 1: the multi-column pull (pull_multi.cuh) over a block of
-// P columns at a time — the row-split schedule, each column folded over
-// the row's entries in ascending order (the reference's `fold`,
-// compute/product/kernel.rs:184-198), long rows split into pieces combined
-// in order — and the write (kernel.rs:200-240) per (row, column).
-template <class E, int S> struct SpmmEpi {
+// SpMM, width > 1: spmm_rows.cuh over a block of P columns at a time, and
+// the write (compute/product/kernel.rs:200-240) per (row, column).
+template <class E, int S, int V> struct SpmmEpi {
   WriteArgs w;
   E* y;
   uint32_t width, c0;
   DeviceError* err;
-  __device__ void cell(uint32_t row, uint32_t c, bool present, E t) {
-    const uint32_t col = c0 + c;
-    if (col >= width) return;
-    E* out = y + (size_t)row * width + col;
+  __device__ void cells(uint32_t row, uint32_t c, bool present, const E (&t)[V]) {
+    E* out = y + (size_t)row * width + c0 + c;
     const E identity = Identity<E>::of(semiring_add(S));
-    if (!mask_selects(w, row)) {
-      if (w.replace) *out = identity;
+    if (V * sizeof(E) == 16 && !w.mask && w.accumulate < 0) {
+      SpmmVec<E, V> r;
+#pragma unroll
+      for (int v = 0; v < V; v++) r.v[v] = present ? t[v] : identity;
+      *reinterpret_cast<SpmmVec<E, V>*>(out) = r;
       return;
     }
-    if (w.accumulate < 0) {
-      *out = present ? t : identity;
-    } else if (present) {
-      E r;
-      int32_t s = apply_rt<E>(w.accumulate, *out, t, &r);
-      if (s) raise(err, s, row);
-      else *out = r;
+    const bool selected = mask_selects(w, row);
+#pragma unroll 1
+    for (int v = 0; v < V; v++) {
+      if (!selected) {
+        if (w.replace) out[v] = identity;
+      } else if (w.accumulate < 0) {
+        out[v] = present ? t[v] : identity;
+      } else if (present) {
+        E r;
+        int32_t s = apply_rt<E>(w.accumulate, out[v], t[v], &r);
+        if (s) raise(err, s, row);
+        else out[v] = r;
+      }
     }
   }
 };
 
+template <class E, int S, class W, int P, int V>
+__global__ void __launch_bounds__(32 * kSpmmWarps, 3)
+    spmm_rows_kernel(CsrView<W> A, const E* __restrict__ x, E* y, uint32_t width, uint32_t c0,
+                     WriteArgs w, DeviceError* err, Partial<E, semiring_add(S)>* carry) {
+  __shared__ SpmmWarp<E> sm[kSpmmWarps];
+  SpmmEpi<E, S, V> epi{w, y, width, c0, err};
+  spmm_rows<E, S, W, P, V>(A, x + c0, epi, err, carry, width, min(P, width - c0),
+                           sm[threadIdx.x >> 5]);
+}
+
+// A lane takes 16 bytes of a row where every row of x and y starts on a
+// 16-byte boundary (and so every block of 32 columns, and every lane's part),
+// else one element; and one element of the types whose accumulator is wide.
+template <class E, int S> constexpr int spmm_vector() {
+  return sizeof(Acc<E, semiring_add(S)>) > 8 || sizeof(E) < 4 ? 1 : 16 / (int)sizeof(E);
+}
+
 template <class E, int S, class W, int P>
-__global__ void __launch_bounds__(256)
-    spmm_multi_kernel(CsrView<W> A, const E* __restrict__ x, E* y, uint32_t width, uint32_t c0,
-                      WriteArgs w, DeviceError* err, Partial<E, semiring_add(S)>* carry) {
-  SpmmEpi<E, S> epi{w, y, width, c0, err};
-  pull_multi<E, S, W, P>(A, x + c0, epi, err, carry, width, min(P, width - c0));
+void launch_spmm(const CsrView<W>& A, const PullLaunch& L, const E* x, E* y, uint32_t c0,
+                 uint32_t blocks) {
+  constexpr int V = spmm_vector<E, S>();
+  auto* carry = static_cast<Partial<E, semiring_add(S)>*>(L.carry_multi);
+  if constexpr (V > 1 && P >= V) {
+    const uintptr_t at = reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y);
+    if (at % 16 == 0 && (size_t)L.width * sizeof(E) % 16 == 0) {
+      note_launch(), spmm_rows_kernel<E, S, W, P, V><<<blocks, 32 * kSpmmWarps, 0, L.stream>>>(
+          A, x, y, L.width, c0, L.write, L.err, carry);
+      return;
+    }
+  }
+  note_launch(), spmm_rows_kernel<E, S, W, P, 1><<<blocks, 32 * kSpmmWarps, 0, L.stream>>>(
+      A, x, y, L.width, c0, L.write, L.err, carry);
 }
 
 template <class E, int S, class W>
@@ -89,28 +121,19 @@ wc_status launch_one(const PullLaunch& L, const void* x, void* y) {
     note_launch(), spmv_pull_kernel<E, S, W><<<blocks, kPullThreads, smem, L.stream>>>(
         A, static_cast<const E*>(x), epi, L.err);
   } else {
-    uint32_t blocks = (L.unit_count + 7) / 8;
+    uint32_t blocks = (L.unit_count + kSpmmWarps - 1) / kSpmmWarps;
     blocks = blocks < 1 ? 1 : (blocks > L.max_blocks ? L.max_blocks : blocks);
-    auto* carry = static_cast<Partial<E, semiring_add(S)>*>(L.carry_multi);
     // Blocks of P columns: P the smallest power of two covering the width,
     // at most 32.
+    const E* xe = static_cast<const E*>(x);
+    E* ye = static_cast<E*>(y);
     for (uint32_t c0 = 0; c0 < L.width; c0 += 32) {
       const uint32_t cols = L.width - c0;
-      if (cols >= 32)
-        note_launch(), spmm_multi_kernel<E, S, W, 32><<<blocks, 256, 0, L.stream>>>(
-            A, static_cast<const E*>(x), static_cast<E*>(y), L.width, c0, L.write, L.err, carry);
-      else if (cols > 8)
-        note_launch(), spmm_multi_kernel<E, S, W, 16><<<blocks, 256, 0, L.stream>>>(
-            A, static_cast<const E*>(x), static_cast<E*>(y), L.width, c0, L.write, L.err, carry);
-      else if (cols > 4)
-        note_launch(), spmm_multi_kernel<E, S, W, 8><<<blocks, 256, 0, L.stream>>>(
-            A, static_cast<const E*>(x), static_cast<E*>(y), L.width, c0, L.write, L.err, carry);
-      else if (cols > 2)
-        note_launch(), spmm_multi_kernel<E, S, W, 4><<<blocks, 256, 0, L.stream>>>(
-            A, static_cast<const E*>(x), static_cast<E*>(y), L.width, c0, L.write, L.err, carry);
-      else
-        note_launch(), spmm_multi_kernel<E, S, W, 2><<<blocks, 256, 0, L.stream>>>(
-            A, static_cast<const E*>(x), static_cast<E*>(y), L.width, c0, L.write, L.err, carry);
+      if (cols > 16) launch_spmm<E, S, W, 32>(A, L, xe, ye, c0, blocks);
+      else if (cols > 8) launch_spmm<E, S, W, 16>(A, L, xe, ye, c0, blocks);
+      else if (cols > 4) launch_spmm<E, S, W, 8>(A, L, xe, ye, c0, blocks);
+      else if (cols > 2) launch_spmm<E, S, W, 4>(A, L, xe, ye, c0, blocks);
+      else launch_spmm<E, S, W, 2>(A, L, xe, ye, c0, blocks);
     }
   }
   return cuda_status(cudaGetLastError(), L.detail, "product kernel launch");
@@ -140,7 +163,9 @@ template <class E>
 wc_status launch_typed(const PullLaunch& L, const void* x, void* y) {
   switch (L.weight_kind) {
     case WEIGHTS_F64: return launch_semiring<E, double>(L, x, y);
-    case WEIGHTS_I32: return launch_semiring<E, int32_t>(L, x, y);
+    case WEIGHTS_I32:  // prepare_pull: the i64 products alone read the i32 copy
+      if constexpr (std::is_same_v<E, int64_t>) return launch_semiring<E, int32_t>(L, x, y);
+      return WC_DTYPE_MISMATCH;
     default: return launch_semiring<E, void>(L, x, y);
   }
 }
