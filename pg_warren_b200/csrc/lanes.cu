@@ -90,6 +90,27 @@ __global__ void lane_bases_kernel(const uint32_t* bases, uint32_t slices, uint32
     units[s].c = first + bases[s];
 }
 
+// Over the nodes: rows of more than `cap` entries (the long ones apart), rows
+// without entries, and nodes gathered often enough for a slot.
+__global__ void lane_counts_kernel(const uint32_t* off, const uint32_t* other, uint32_t n,
+                                   uint32_t cap, uint32_t* counts) {
+  uint32_t wide = 0, empty = 0, hot = 0;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const uint32_t deg = off[i + 1] - off[i];
+    wide += deg > cap && deg <= kPieceEntries;
+    empty += deg == 0;
+    hot += other[i + 1] - other[i] >= kHotGathers;
+  }
+  wide = __reduce_add_sync(0xffffffffu, wide);
+  empty = __reduce_add_sync(0xffffffffu, empty);
+  hot = __reduce_add_sync(0xffffffffu, hot);
+  if ((threadIdx.x & 31) == 0) {
+    if (wide) atomicAdd(counts, wide);
+    if (empty) atomicAdd(counts + 1, empty);
+    if (hot) atomicAdd(counts + 2, hot);
+  }
+}
+
 __global__ void hot_slots_kernel(const uint32_t* hot, uint32_t count, uint32_t* slot_of) {
   const uint32_t h = blockIdx.x * blockDim.x + threadIdx.x;
   if (h < count) slot_of[hot[h]] = kHotTarget | h;
@@ -135,8 +156,7 @@ __global__ void lane_entries_kernel(const LaneUnit* units, uint32_t count, const
 }
 
 wc_status device_lanes(wc_version* v, DevCsr& d, const std::vector<uint64_t>& off,
-                       const DevCsr& other, const std::vector<uint64_t>& other_off,
-                       wc_error_detail* detail) {
+                       const DevCsr& other, wc_error_detail* detail) {
   const uint64_t n = v->n, m = v->m;
   cudaStream_t st = v->stream;
   LaneCsr& L = d.lanes;
@@ -151,25 +171,32 @@ wc_status device_lanes(wc_version* v, DevCsr& d, const std::vector<uint64_t>& of
   uint64_t cap = 32;
   while (cap < kPieceEntries && m / 32 >= 2 * (2 * cap) * kLaneWarps) cap *= 2;
   std::vector<LaneUnit> groups;
-  uint64_t long_entries = 0, hot_nodes = 0;
-  uint32_t slot = 0, empty = 0;
-  LaneClasses cls{};
-  for (uint64_t r = 0; r < n; r++) {
-    const uint64_t deg = off[r + 1] - off[r];
-    if (other_off[r + 1] - other_off[r] >= kHotGathers) hot_nodes++;
-    if (deg <= kPieceEntries) {
-      if (!deg) empty++;
-      cls.row[1] += deg > cap;
-      continue;
-    }
-    long_entries += deg;
-    const uint32_t pieces = (uint32_t)((deg + kPieceEntries - 1) / kPieceEntries);
-    for (uint32_t f = 0; f < pieces; f += run)
-      groups.push_back(LaneUnit{(uint32_t)r, f << 8 | std::min(run, pieces - f),
-                                (slot + f) * (kPieceEntries / 32), 1u << 31 | slot});
-    slot += pieces;
+  std::vector<uint4> longs(d.schedule.long_rows);  // row, first slot, pieces
+  uint32_t counts[3] = {0, 0, 0};
+  DevBuf tally;
+  WC_TRY(tally.alloc(v->budget, sizeof counts, detail));
+  WC_CUDA(cudaMemsetAsync(tally.ptr, 0, sizeof counts, st), detail);
+  if (n)
+    note_launch(), lane_counts_kernel<<<grid_of(n), 256, 0, st>>>(
+        d.offsets.as<uint32_t>(), other.offsets.as<uint32_t>(), (uint32_t)n, (uint32_t)cap,
+        tally.as<uint32_t>());
+  WC_CUDA(cudaMemcpyAsync(counts, tally.ptr, sizeof counts, cudaMemcpyDeviceToHost, st), detail);
+  if (!longs.empty())
+    WC_CUDA(cudaMemcpyAsync(longs.data(), d.schedule.long_list.ptr, longs.size() * sizeof(uint4),
+                            cudaMemcpyDeviceToHost, st), detail);
+  WC_CUDA(cudaStreamSynchronize(st), detail);
+  uint64_t long_entries = 0;
+  const uint32_t slot = d.schedule.slots;
+  for (const uint4& l : longs) {
+    long_entries += off[l.x + 1] - off[l.x];
+    for (uint32_t f = 0; f < l.z; f += run)
+      groups.push_back(LaneUnit{l.x, f << 8 | std::min(run, l.z - f),
+                                (l.y + f) * (kPieceEntries / 32), 1u << 31 | l.y});
   }
-  cls.row[2] = L.filled = shorts - empty;
+  LaneClasses cls{};
+  const uint64_t hot_nodes = counts[2];
+  cls.row[1] = counts[0];
+  cls.row[2] = L.filled = shorts - counts[1];
   L.shorts = shorts;
   for (uint32_t q = 0; q < 2; q++) {
     const uint32_t per = q ? 32 : 32 / kWideLanes;
@@ -192,23 +219,34 @@ wc_status device_lanes(wc_version* v, DevCsr& d, const std::vector<uint64_t>& of
   if (d.iweights.ptr) WC_TRY(L.iweights.alloc(v->budget, places * 4, detail));
   if (L.hot_count) WC_TRY(L.hot.alloc(v->budget, L.hot_count * 4, detail));
   if (!n) return WC_OK;
-  DevBuf keys, ids, temp;  // keys, then (n words) the second key buffer
-  WC_TRY(keys.alloc(v->budget, 2 * n * 4, detail));
-  WC_TRY(ids.alloc(v->budget, std::max<uint64_t>(n, 2 * slices) * 4, detail));
-  uint32_t* k0 = keys.as<uint32_t>();
-  size_t temp_bytes = 0, scan_bytes = 0;
-  cub::DoubleBuffer<uint32_t> kb(k0, k0 + n);
-  cub::DoubleBuffer<uint32_t> ib(L.rows.as<uint32_t>(), ids.as<uint32_t>());
-  WC_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, temp_bytes, kb, ib, (int)n, 0, 32, st), detail);
-  WC_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, k0, k0, (int)slices, st), detail);
-  WC_TRY(temp.alloc(v->budget, std::max<size_t>({temp_bytes, scan_bytes, 16}), detail));
+  // One transient buffer: two key and two id buffers of n words, the sorts'
+  // and the scan's temporary memory behind them.  (The rows are sorted into
+  // place by a copy.)
+  size_t sort_bytes = 0, scan_bytes = 0;
+  {
+    cub::DoubleBuffer<uint32_t> none(nullptr, nullptr);
+    uint32_t* nowhere = nullptr;
+    WC_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, none, none, (int)n, 0, 32, st),
+            detail);
+    WC_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, nowhere, nowhere, (int)slices, st),
+            detail);
+  }
+  const uint64_t words = (n + 63) / 64 * 64, ids_at = 2 * words;
+  const uint64_t temp_at = (ids_at + std::max<uint64_t>(words, 2 * slices) + 63) / 64 * 64;
+  size_t temp_bytes = std::max<size_t>({sort_bytes, scan_bytes, 16});
+  DevBuf transient;
+  WC_TRY(transient.alloc(v->budget, temp_at * 4 + temp_bytes, detail));
+  uint32_t* k0 = transient.as<uint32_t>();
+  uint32_t* ids = k0 + ids_at;
+  void* temp = k0 + temp_at;
+  cub::DoubleBuffer<uint32_t> kb(k0, k0 + words);
+  cub::DoubleBuffer<uint32_t> ib(L.rows.as<uint32_t>(), ids);
   // The hot nodes: the front of the nodes sorted by gathers.
   uint32_t* slot_of = nullptr;
   if (L.hot_count) {
     note_launch(), gather_keys_kernel<<<grid_of(n), 256, 0, st>>>(
         other.offsets.as<uint32_t>(), (uint32_t)n, kb.Current(), ib.Current());
-    temp_bytes = temp.bytes;
-    WC_CUDA(cub::DeviceRadixSort::SortPairs(temp.ptr, temp_bytes, kb, ib, (int)n, 0, 32, st),
+    WC_CUDA(cub::DeviceRadixSort::SortPairs(temp, temp_bytes, kb, ib, (int)n, 0, 32, st),
             detail);
     WC_CUDA(cudaMemcpyAsync(L.hot.ptr, ib.Current(), L.hot_count * 4, cudaMemcpyDeviceToDevice, st),
             detail);
@@ -216,22 +254,20 @@ wc_status device_lanes(wc_version* v, DevCsr& d, const std::vector<uint64_t>& of
   // The short rows, longest first.
   note_launch(), lane_keys_kernel<<<grid_of(n), 256, 0, st>>>(
       d.offsets.as<uint32_t>(), (uint32_t)n, kb.Current(), ib.Current());
-  temp_bytes = temp.bytes;
-  WC_CUDA(cub::DeviceRadixSort::SortPairs(temp.ptr, temp_bytes, kb, ib, (int)n, 0, 9, st), detail);
+  WC_CUDA(cub::DeviceRadixSort::SortPairs(temp, temp_bytes, kb, ib, (int)n, 0, 9, st), detail);
   if (ib.Current() != L.rows.as<uint32_t>())
     WC_CUDA(cudaMemcpyAsync(L.rows.ptr, ib.Current(), n * 4, cudaMemcpyDeviceToDevice, st), detail);
   if (!groups.empty())
     WC_CUDA(cudaMemcpyAsync(L.units.ptr, groups.data(), groups.size() * sizeof(LaneUnit),
                             cudaMemcpyHostToDevice, st), detail);
   if (slices) {
-    uint32_t *steps = ids.as<uint32_t>(), *bases = steps + slices;
+    uint32_t *steps = ids, *bases = steps + slices;
     LaneUnit* units = L.units.as<LaneUnit>() + groups.size();
     note_launch(), lane_lengths_kernel<<<grid_of(shorts), 256, 0, st>>>(
         d.offsets.as<uint32_t>(), L.rows.as<uint32_t>(), shorts, L.lengths.as<uint16_t>());
     note_launch(), lane_slices_kernel<<<grid_of(slices), 256, 0, st>>>(
         cls, L.lengths.as<uint16_t>(), units, steps);
-    temp_bytes = temp.bytes;
-    WC_CUDA(cub::DeviceScan::ExclusiveSum(temp.ptr, temp_bytes, steps, bases, (int)slices, st),
+    WC_CUDA(cub::DeviceScan::ExclusiveSum(temp, temp_bytes, steps, bases, (int)slices, st),
             detail);
     note_launch(), lane_bases_kernel<<<grid_of(slices), 256, 0, st>>>(bases, slices, first, units);
   }

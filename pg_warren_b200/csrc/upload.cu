@@ -54,6 +54,57 @@ __global__ void unpack_sources_kernel(const uint64_t* keys, uint64_t m, uint32_t
     rtgt[e] = (uint32_t)keys[e];
 }
 
+// The position of the first target outside the id space (m: none).
+__global__ void outside_kernel(const uint32_t* tgt, uint64_t m, uint32_t n,
+                               unsigned long long* first) {
+  unsigned long long mine = m;
+  for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < m;
+       e += (uint64_t)gridDim.x * blockDim.x)
+    if (tgt[e] >= n && e < mine) mine = e;
+  if (mine < m) atomicMin(first, mine);
+}
+
+wc_status device_targets_in_space(wc_version* v, wc_error_detail* detail) {
+  if (!v->m) return WC_OK;
+  DevBuf first;
+  WC_TRY(first.alloc(v->budget, 8, detail));
+  unsigned long long at = v->m;
+  WC_CUDA(cudaMemcpyAsync(first.ptr, &at, 8, cudaMemcpyHostToDevice, v->stream), detail);
+  note_launch(), outside_kernel<<<max_blocks(8), 256, 0, v->stream>>>(
+      v->fwd.targets.as<uint32_t>(), v->m, (uint32_t)v->n, first.as<unsigned long long>());
+  WC_CUDA(cudaMemcpyAsync(&at, first.ptr, 8, cudaMemcpyDeviceToHost, v->stream), detail);
+  WC_CUDA(cudaStreamSynchronize(v->stream), detail);
+  if (at == v->m) return WC_OK;
+  uint32_t target = 0;
+  WC_CUDA(cudaMemcpy(&target, v->fwd.targets.as<uint32_t>() + at, 4, cudaMemcpyDeviceToHost),
+          detail);
+  if (detail) detail->node = target;
+  return WC_NODE_OUTSIDE_ID_SPACE;
+}
+
+__global__ void row_masks_kernel(const Unit* units, uint32_t count, const uint32_t* off,
+                                 uint32_t* masks) {
+  const uint32_t lane = threadIdx.x & 31;
+  const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+  for (uint32_t u = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; u < count; u += warps) {
+    const Unit d = units[u];
+    const bool piece = d.c >> 31;
+    const uint32_t r = d.a + lane;
+    const bool holds = piece ? lane == 0 : r < d.b && off[r + 1] > off[r];
+    const uint32_t mask = __ballot_sync(0xffffffffu, holds);
+    if (lane == 0) masks[u] = mask;
+  }
+}
+
+wc_status device_row_masks(wc_version* v, DevCsr& d, wc_error_detail* detail) {
+  const uint32_t count = d.schedule.count;
+  if (count)
+    note_launch(), row_masks_kernel<<<max_blocks(8), 256, 0, v->stream>>>(
+        d.schedule.units.as<Unit>(), count, d.offsets.as<uint32_t>(),
+        d.schedule.row_masks.as<uint32_t>());
+  return cuda_status(cudaStreamSynchronize(v->stream), detail, "row masks");
+}
+
 // ---------------------------------------------------------- weight facts
 
 // Whether every weight is an integer in i32 range (an exact i32 copy is then

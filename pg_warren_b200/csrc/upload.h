@@ -14,6 +14,11 @@ wc_status wc_device_check(wc_error_detail* detail);
 // The reverse CSR from the forward one, on the device (v->rev, and its
 // offsets on the host).
 wc_status device_reverse(wc_version* v, wc_error_detail* detail);
+// Every target of the forward CSR against the id space, on the device: the
+// first outside it is WC_NODE_OUTSIDE_ID_SPACE with the target in the detail.
+wc_status device_targets_in_space(wc_version* v, wc_error_detail* detail);
+// The schedule's per-unit masks of the rows that hold entries.
+wc_status device_row_masks(wc_version* v, DevCsr& d, wc_error_detail* detail);
 // Whether every weight is an i32 integer (then i32 copies of both
 // orientations' weights) and the largest magnitude.
 wc_status device_weight_facts(wc_version* v, wc_error_detail* detail);
@@ -28,10 +33,9 @@ wc_status put_schedule(wc_version* v, DevCsr& d, const std::vector<uint64_t>& of
                        wc_error_detail* detail);
 // The lane-major copy of `d` (v->fwd or v->rev), after its schedule: `off`
 // are its host offsets, `other` the other orientation (whose row lengths say
-// how often each node is gathered) and `other_off` its host offsets.
+// how often each node is gathered).
 wc_status device_lanes(wc_version* v, DevCsr& d, const std::vector<uint64_t>& off,
-                       const DevCsr& other, const std::vector<uint64_t>& other_off,
-                       wc_error_detail* detail);
+                       const DevCsr& other, wc_error_detail* detail);
 // The reverse CSR in locality order (v->loc), after the weights' facts.
 wc_status device_locality(wc_version* v, wc_error_detail* detail);
 // Vectors between dense ids and the locality numbering, on `st`:

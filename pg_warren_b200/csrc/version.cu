@@ -119,20 +119,8 @@ wc_status put_schedule(wc_version* v, DevCsr& d, const std::vector<uint64_t>& of
     WC_CUDA(cudaMemcpy(s.long_list.ptr, longs.data(), longs.size() * 4, cudaMemcpyHostToDevice),
             detail);
   // Per tile, its rows that hold entries (a piece's row always does).
-  std::vector<uint32_t> masks(units.size(), 1u);
-  for (size_t u = 0; u < units.size(); u++) {
-    const Unit& d = units[u];
-    if ((d.c >> 31) != 0) continue;
-    uint32_t m = 0;
-    for (uint32_t r = d.a; r < d.b; r++)
-      if (off[r + 1] > off[r]) m |= 1u << (r - d.a);
-    masks[u] = m;
-  }
-  WC_TRY(s.row_masks.alloc(v->budget, std::max<size_t>(masks.size(), 1) * 4, detail));
-  if (!masks.empty())
-    WC_CUDA(cudaMemcpy(s.row_masks.ptr, masks.data(), masks.size() * 4, cudaMemcpyHostToDevice),
-            detail);
-  return WC_OK;
+  WC_TRY(s.row_masks.alloc(v->budget, std::max<size_t>(units.size(), 1) * 4, detail));
+  return device_row_masks(v, d, detail);
 }
 
 wc_status wc_device_check(wc_error_detail* detail) {
@@ -158,8 +146,8 @@ wc_status finish_version(wc_version* v, wc_error_detail* detail) {
   WC_TRY(device_symmetric(v, detail));
   WC_TRY(put_schedule(v, v->fwd, v->host_offsets, detail));
   WC_TRY(put_schedule(v, v->rev, v->host_rev_offsets, detail));
-  WC_TRY(device_lanes(v, v->fwd, v->host_offsets, v->rev, v->host_rev_offsets, detail));
-  WC_TRY(device_lanes(v, v->rev, v->host_rev_offsets, v->fwd, v->host_offsets, detail));
+  WC_TRY(device_lanes(v, v->fwd, v->host_offsets, v->rev, detail));
+  WC_TRY(device_lanes(v, v->rev, v->host_rev_offsets, v->fwd, detail));
   WC_TRY(device_locality(v, detail));
   WC_TRY(v->error.alloc(v->budget, sizeof(DeviceError), detail));
   WC_CUDA(cudaMemset(v->error.ptr, 0, sizeof(DeviceError)), detail);
@@ -255,11 +243,6 @@ wc_status wc_version_upload(uint64_t graph_id, uint64_t version, const wc_csr_ho
   WC_TRY(wc_device_check(detail));
   const uint64_t n = csr->id_space, m = csr->edges;
   if (csr->offsets[0] != 0 || csr->offsets[n] != m) return WC_INVALID_ARGUMENT;
-  for (uint64_t e = 0; e < m; e++)
-    if (csr->targets[e] >= n) {
-      if (detail) detail->node = csr->targets[e];
-      return WC_NODE_OUTSIDE_ID_SPACE;
-    }
   if (csr->reverse_offsets && (!csr->reverse_targets || (csr->weights && !csr->reverse_weights)))
     return WC_INVALID_ARGUMENT;
   std::unique_ptr<wc_version> v(new wc_version);
@@ -273,6 +256,10 @@ wc_status wc_version_upload(uint64_t graph_id, uint64_t version, const wc_csr_ho
   WC_CUDA(cudaGetDevice(&v->device), detail);
   WC_CUDA(cudaStreamCreateWithFlags(&v->stream, cudaStreamNonBlocking), detail);
   WC_TRY(put_csr(v.get(), v->fwd, csr->offsets, csr->targets, csr->weights, detail));
+  if (const wc_status outside = device_targets_in_space(v.get(), detail)) {
+    cudaStreamDestroy(v->stream);
+    return outside;
+  }
   v->host_offsets.assign(csr->offsets, csr->offsets + n + 1);
   // The reverse CSR: the caller's, or a transpose on the device.
   if (csr->reverse_offsets) {
