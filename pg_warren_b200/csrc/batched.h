@@ -38,6 +38,7 @@ wc_status bfs_batched_run(Ctx& ctx, const wc_schedule& sched, const uint64_t* so
 // columns, sources / caps / the call's column of each in device memory.
 typedef wc_status (*Mp32Fn)(Ctx&, const uint64_t*, const uint32_t*, const uint32_t*, uint32_t,
                             uint32_t, int64_t*, uint32_t*, uint32_t);
+constexpr uint32_t kMp32Blocks = 5;  // of four warps, an SM (batched_minplus32.cu)
 Mp32Fn mp32_for(uint32_t columns);
 wc_status mp32_reserve(Ctx& ctx, uint32_t columns);
 

@@ -7,8 +7,7 @@
 // plus) maps to i32::MAX: the distances and the per-column iteration counts
 // are the i64 loop's.
 //
-// A pass runs P = 32 or 64 columns; a row's P distances are spread over
-// LPR = P/4 lanes holding four each (16-byte accesses).  An iteration reads
+// A pass runs P = 32 or 64 columns, P / 32 a lane.  An iteration reads
 // the previous iterate only (next = min(x, Aᵀ ⊗ x)); after iteration t every
 // row holds x_i ≤ x_j + w for the values of iteration t-1, so iteration t+1
 // folds only the entries whose source row fell at t (a bitmap).  Rows that
@@ -20,6 +19,7 @@
 
 #include "batched.h"
 #include "operand.h"
+#include "pull.cuh"
 #include "semiring.cuh"
 
 namespace wc {
@@ -48,12 +48,26 @@ struct Mp32 {
 
 __device__ inline int32_t add_absorbing(int32_t x, int32_t w) { return x == kInf32 ? kInf32 : x + w; }
 
-template <int P> struct Mp32Smem {
-  int32_t acc[32 * P];
-  uint32_t hitj[kTileEntries];
-  int32_t hitw[kTileEntries];
-  uint8_t hitr[kTileEntries];
-  uint8_t rowof[kTileEntries];
+constexpr uint32_t kMp32Warps = 4;    // warps a block
+constexpr uint32_t kMp32Rows = 16;    // rows whose minima wait to be settled
+constexpr uint32_t kMp32Unroll = 16;  // entries gathered at once
+
+// A lane's columns of a row.
+template <int C> struct alignas(4 * C) Cols32 { int32_t v[C]; };
+
+__device__ inline Cols32<1> load_cols(const Cols32<1>* p) {
+  return Cols32<1>{{__ldg(p->v)}};
+}
+__device__ inline Cols32<2> load_cols(const Cols32<2>* p) {
+  const int2 v = __ldg(reinterpret_cast<const int2*>(p));
+  return Cols32<2>{{v.x, v.y}};
+}
+
+// A warp's shared memory: the unit's hits and the rows' minima.
+template <int P> struct Mp32Warp {
+  Cols32<P / 32> y[kMp32Rows][32];
+  uint32_t j[kTileEntries];
+  int32_t w[kTileEntries];
 };
 
 __global__ void mp32_fill_kernel(int32_t* p, uint64_t count, int32_t v) {
@@ -95,180 +109,180 @@ __global__ void mp32_sources_kernel(Mp32 s, const uint64_t* sources) {
   }
 }
 
-// One iteration over the reverse CSR's schedule.
+// One iteration over the reverse CSR's schedule: a warp per unit, a row of x
+// the warp's 32 lanes.  The unit's hits (entries whose source row fell) are
+// listed in shared memory, gathered sixteen at a time whatever rows they
+// belong to, and folded row by row; the tile's rows that had hits are settled
+// four at a time.  Bound by the latency of the row gathers (256 bytes a hit
+// out of L2): sixteen rows in flight a warp, twenty warps an SM, where the
+// kernel that kept per-row minima in shared memory had two half-warps' eight
+// in flight in sixteen warps.
 template <int P>
-__global__ void __launch_bounds__(256, 3) mp32_iter_kernel(Mp32 s, uint32_t it) {
-  constexpr uint32_t LPR = P / 4;       // lanes a row
-  constexpr uint32_t G = 32 / LPR;      // rows (or gathered rows) a warp instruction covers
-  constexpr uint32_t GM = LPR == 32 ? 0xffffffffu : (1u << LPR) - 1;
+__global__ void __launch_bounds__(32 * kMp32Warps, 5) mp32_iter_kernel(Mp32 s, uint32_t it) {
+  constexpr int C = P / 32;
   constexpr int Q = kTileEntries / 32;
-  constexpr int U = 8;
-  constexpr uint32_t VR = kTileRows / G;
-  bool any_running = false;
-  for (uint32_t q = 0; q < P / 32; q++) any_running |= s.running[q] != 0;
+  constexpr uint32_t U = kMp32Unroll;
+  typedef Cols32<C> Cols;
+  uint32_t running[C], any_running = 0;
+#pragma unroll
+  for (int c = 0; c < C; c++) any_running |= running[c] = s.running[c];
   if (!any_running) return;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  Mp32Smem<P>& sm = reinterpret_cast<Mp32Smem<P>*>(smem_raw)[threadIdx.x >> 5];
+  __shared__ Mp32Warp<P> sm_all[kMp32Warps];
+  Mp32Warp<P>& sm = sm_all[threadIdx.x >> 5];
   const unsigned lane = threadIdx.x & 31;
-  const unsigned sub = lane / LPR, q = lane % LPR;
-  const uint32_t c0 = q * 4;  // this lane's four columns
-  const unsigned gmask = GM << (sub * LPR);
-  const uint32_t run4 = (s.running[c0 >> 5] >> (c0 & 31)) & 0xFu;  // running bits of c0..c0+3
+  // The lane's columns C·lane .. C·lane + C - 1: which of them still run.
+  uint32_t run = 0;
+#pragma unroll
+  for (int c = 0; c < C; c++) {
+    const uint32_t col = C * lane + c;
+    run |= ((running[C == 1 ? 0 : col >> 5] >> (col & 31)) & 1u) << c;
+  }
   const uint32_t* fell_cur = s.fell_rows[it & 1];
   uint32_t* fell_next = s.fell_rows[(it + 1) & 1];
+  const Cols* x = reinterpret_cast<const Cols*>(s.x) + lane;
+  Cols* next = reinterpret_cast<Cols*>(s.next) + lane;
   const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-  uint32_t fell_cols = 0;  // bits of this lane's four columns that fell
+  uint32_t fell_cols = 0;  // bits of this lane's columns that fell
+  Cols none;
+#pragma unroll
+  for (int c = 0; c < C; c++) none.v[c] = kInf32;
 
-  // new = min(old, got) for running columns; f: the columns that fell.
-  auto settle = [&](uint32_t i, const int4& got, int4& nv) -> uint32_t {
-    const int4 old = *reinterpret_cast<const int4*>(s.x + (size_t)i * P + c0);
-    nv = old;
-    if ((run4 & 1) && got.x < old.x) nv.x = got.x;
-    if ((run4 & 2) && got.y < old.y) nv.y = got.y;
-    if ((run4 & 4) && got.z < old.z) nv.z = got.z;
-    if ((run4 & 8) && got.w < old.w) nv.w = got.w;
-    return (nv.x < old.x ? 1u : 0u) | (nv.y < old.y ? 2u : 0u) | (nv.z < old.z ? 4u : 0u) |
-           (nv.w < old.w ? 8u : 0u);
+  // Row i's new values where a running column's minimum is below the old one.
+  auto settle = [&](uint32_t i, const Cols& got, const Cols& old) {
+    Cols nv = old;
+    uint32_t f = 0;
+#pragma unroll
+    for (int c = 0; c < C; c++)
+      if (((run >> c) & 1) && got.v[c] < old.v[c]) {
+        nv.v[c] = got.v[c];
+        f |= 1u << c;
+      }
+    if (__any_sync(0xffffffffu, f != 0)) {
+      next[(size_t)i * 32] = nv;
+      if (lane == 0) atomicOr(fell_next + (i >> 5), 1u << (i & 31));
+    }
+    fell_cols |= f;
   };
 
+  Unit ahead{};
+  if (warp < s.unit_count) ahead = s.units[warp];
   for (uint32_t u = warp; u < s.unit_count; u += warps) {
-    const Unit unit = s.units[u];
+    const Unit unit = ahead;
+    if (u + warps < s.unit_count) {
+      ahead = s.units[u + warps];
+      if (32 * lane < unit_count(ahead))  // its targets into L2 meanwhile
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(s.tgt + unit_first(ahead) + 32 * lane));
+    }
     const bool tile = (unit.c >> 31) == 0;
-    const uint32_t r0 = unit.a;
     const uint32_t R = tile ? unit.b - unit.a : 1;
-    uint32_t base, count;
-    if (tile) {
-      uint32_t lo = 0, hi = 0;
-      if (lane < R) {
-        lo = __ldg(s.off + r0 + lane);
-        hi = __ldg(s.off + r0 + lane + 1);
-      }
-      base = unit.d;
-      count = unit.c;
-      for (uint32_t k = lo - base; k < hi - base; k++) sm.rowof[k] = (uint8_t)lane;
-      for (uint32_t x = lane * 4; x < R * P; x += 128)
-        *reinterpret_cast<int4*>(&sm.acc[x]) = make_int4(kInf32, kInf32, kInf32, kInf32);
-    } else {
-      base = unit.b;
-      count = unit.d - unit.b;
-    }
-    __syncwarp();
+    const uint32_t base = unit_first(unit), count = unit_count(unit);
+    __syncwarp();  // every lane is done with the last unit's shared memory
     // The hits: entries whose source row fell in the previous iteration.
-    uint32_t H = 0;
-    {
-      uint32_t jv[Q];
+    uint32_t jv[Q], mask[Q], H = 0;
 #pragma unroll
-      for (int qq = 0; qq < Q; qq++) {
-        const uint32_t k = lane + 32 * qq;
-        jv[qq] = k < count ? __ldcs(s.tgt + base + k) : 0u;
-      }
+    for (int q = 0; q < Q; q++) {
+      const uint32_t k = lane + 32 * q;
+      jv[q] = k < count ? __ldcs(s.tgt + base + k) : 0u;
+    }
+    uint32_t end_l = count;  // the lane's row's end
+    if (tile && lane < R) end_l = __ldg(s.off + unit.a + lane + 1) - base;
 #pragma unroll
-      for (int qq = 0; qq < Q; qq++) {
-        const uint32_t k = lane + 32 * qq;
-        const bool hit = k < count && ((fell_cur[jv[qq] >> 5] >> (jv[qq] & 31)) & 1);
-        const uint32_t m = __ballot_sync(0xffffffffu, hit);
-        if (hit) {
-          const uint32_t pos = H + __popc(m & ((1u << lane) - 1));
-          sm.hitj[pos] = jv[qq];
-          sm.hitw[pos] = s.w ? __ldg(s.w + base + k) : 1;
-          sm.hitr[pos] = tile ? sm.rowof[k] : (uint8_t)0;
-        }
-        H += __popc(m);
+    for (int q = 0; q < Q; q++) {
+      const uint32_t k = lane + 32 * q;
+      const bool hit = k < count && ((__ldg(fell_cur + (jv[q] >> 5)) >> (jv[q] & 31)) & 1);
+      mask[q] = __ballot_sync(0xffffffffu, hit);
+      if (hit) {
+        const uint32_t at = H + __popc(mask[q] & ((1u << lane) - 1));
+        sm.j[at] = jv[q];
+        sm.w[at] = s.w ? __ldg(s.w + base + k) : 1;
       }
+      H += __popc(mask[q]);
+    }
+    if (!H && tile) continue;  // no row of the tile can fall
+    // The hits before the lane's row's end.
+    uint32_t hi_l = 0;
+#pragma unroll
+    for (int q = 0; q < Q; q++) {
+      const uint32_t from = 32 * q;
+      hi_l += end_l >= from + 32 ? __popc(mask[q])
+              : end_l > from     ? __popc(mask[q] & ((1u << (end_l - from)) - 1))
+                                 : 0;
     }
     __syncwarp();
-    // Gather: group g takes hits [g·H/G, (g+1)·H/G) in order; a row's hits
-    // are consecutive, so their minima stay in registers until the row
-    // changes.
-    int4 run = make_int4(kInf32, kInf32, kInf32, kInf32);
-    if (H) {
-      const uint32_t per = (H + G - 1) / G;
-      const uint32_t h_lo = min(H, sub * per), h_hi = min(H, sub * per + per);
-      uint32_t cur = h_lo < h_hi ? sm.hitr[h_lo] : 0u;
-      for (uint32_t h0 = h_lo; h0 < h_hi; h0 += U) {
-        int4 val[U];
-        int32_t wv[U];
-        uint32_t rr[U];
+    Cols acc = none;
+    auto gather = [&](uint32_t k) { return load_cols(x + (size_t)sm.j[k] * 32); };
+    auto fold = [&](uint32_t k, const Cols& v) {
+      const int32_t w = sm.w[k];
 #pragma unroll
-        for (int x = 0; x < U; x++) {
-          const uint32_t h = h0 + x;
-          rr[x] = cur;
-          wv[x] = 0;
-          val[x] = make_int4(kInf32, kInf32, kInf32, kInf32);
-          if (h < h_hi) {
-            val[x] = __ldg(reinterpret_cast<const int4*>(s.x + (size_t)sm.hitj[h] * P + c0));
-            wv[x] = sm.hitw[h];
-            rr[x] = sm.hitr[h];
-          }
+      for (int c = 0; c < C; c++) acc.v[c] = min(acc.v[c], add_absorbing(v.v[c], w));
+    };
+    uint32_t k = 0;
+    for (uint32_t r0 = 0; r0 < R; r0 += kMp32Rows) {
+      const uint32_t r1 = min(R, r0 + kMp32Rows);
+      const uint32_t end = __shfl_sync(0xffffffffu, hi_l, r1 - 1);
+      uint32_t lo = k;  // the hits before row r0
+      uint32_t r = r0;
+      uint32_t hi = __shfl_sync(0xffffffffu, hi_l, r);
+      auto close = [&](uint32_t at) {
+        while (at == hi && r < r1) {
+          sm.y[r - r0][lane] = acc;
+          acc = none;
+          r++;
+          hi = __shfl_sync(0xffffffffu, hi_l, r & 31);
         }
+      };
+      for (; k < end; k += U) {
+        Cols v[U];
+        const uint32_t n = min(U, end - k);
 #pragma unroll
-        for (int x = 0; x < U; x++) {
-          if (rr[x] != cur) {
-            if (tile) {
-              int32_t* a = &sm.acc[cur * P + c0];
-              if (run.x != kInf32) atomicMin(a, run.x);
-              if (run.y != kInf32) atomicMin(a + 1, run.y);
-              if (run.z != kInf32) atomicMin(a + 2, run.z);
-              if (run.w != kInf32) atomicMin(a + 3, run.w);
+        for (uint32_t q = 0; q < U; q++)
+          if (q < n) v[q] = gather(k + q);
+        if (!tile || (k < hi && k + n <= hi)) {
+#pragma unroll
+          for (uint32_t q = 0; q < U; q++)
+            if (q < n) fold(k + q, v[q]);
+        } else {
+#pragma unroll
+          for (uint32_t q = 0; q < U; q++)
+            if (q < n) {
+              if (k + q == hi) close(k + q);
+              fold(k + q, v[q]);
             }
-            run = make_int4(kInf32, kInf32, kInf32, kInf32);
-            cur = rr[x];
-          }
-          run.x = min(run.x, add_absorbing(val[x].x, wv[x]));
-          run.y = min(run.y, add_absorbing(val[x].y, wv[x]));
-          run.z = min(run.z, add_absorbing(val[x].z, wv[x]));
-          run.w = min(run.w, add_absorbing(val[x].w, wv[x]));
         }
       }
-      if (tile) {
-        int32_t* a = &sm.acc[cur * P + c0];
-        if (run.x != kInf32) atomicMin(a, run.x);
-        if (run.y != kInf32) atomicMin(a + 1, run.y);
-        if (run.z != kInf32) atomicMin(a + 2, run.z);
-        if (run.w != kInf32) atomicMin(a + 3, run.w);
+      k = end;
+      if (!tile) break;
+      close(k);
+      for (uint32_t e = r0; e < r1; e += 4) {
+        Cols old[4];
+        uint32_t had = 0, upto = lo;
+#pragma unroll
+        for (uint32_t q = 0; q < 4; q++) {
+          const uint32_t h = __shfl_sync(0xffffffffu, hi_l, (e + q) & 31);
+          if (e + q < r1 && h > upto) {
+            had |= 1u << q;
+            old[q] = x[(size_t)(unit.a + e + q) * 32];
+          }
+          if (e + q < r1) upto = h;
+        }
+#pragma unroll
+        for (uint32_t q = 0; q < 4; q++)
+          if ((had >> q) & 1) settle(unit.a + e + q, sm.y[e + q - r0][lane], old[q]);
+        lo = upto;
       }
     }
-    __syncwarp();
-    if (tile) {
-#pragma unroll
-      for (uint32_t x = 0; x < VR; x++) {
-        if (x * G >= R) break;
-        const uint32_t r = x * G + sub;
-        uint32_t f = 0;
-        int4 nv = make_int4(0, 0, 0, 0);
-        if (r < R) {
-          const int4 got = *reinterpret_cast<const int4*>(&sm.acc[r * P + c0]);
-          f = settle(r0 + r, got, nv);
-        }
-        if (__ballot_sync(0xffffffffu, f != 0) & gmask) {
-          *reinterpret_cast<int4*>(s.next + (size_t)(r0 + r) * P + c0) = nv;
-          if (q == 0) atomicOr(fell_next + ((r0 + r) >> 5), 1u << ((r0 + r) & 31));
-        }
-        fell_cols |= f;
-      }
-      __syncwarp();
-    } else {
-      // The groups' minima, then into the row's global accumulator.
-#pragma unroll
-      for (uint32_t o = LPR; o < 32; o <<= 1) {
-        run.x = min(run.x, __shfl_xor_sync(0xffffffffu, run.x, o));
-        run.y = min(run.y, __shfl_xor_sync(0xffffffffu, run.y, o));
-        run.z = min(run.z, __shfl_xor_sync(0xffffffffu, run.z, o));
-        run.w = min(run.w, __shfl_xor_sync(0xffffffffu, run.w, o));
-      }
+    if (!tile) {
+      // A piece's minima into the row's global accumulator.
       const uint32_t row = unit.a, slot = unit.c & 0x7fffffffu;
       const uint32_t row_lo = __ldg(s.off + row);
       const uint32_t deg = __ldg(s.off + row + 1) - row_lo;
       const uint32_t pieces = (deg + kPieceEntries - 1) / kPieceEntries;
-      const uint32_t first = slot - (unit.b - row_lo) / kPieceEntries;
-      int32_t* na = s.nacc + (size_t)first * P + c0;
-      if (sub == 0) {
-        if (run.x != kInf32) atomicMin(na, run.x);
-        if (run.y != kInf32) atomicMin(na + 1, run.y);
-        if (run.z != kInf32) atomicMin(na + 2, run.z);
-        if (run.w != kInf32) atomicMin(na + 3, run.w);
-      }
+      const uint32_t first = slot - (base - row_lo) / kPieceEntries;
+      int32_t* na = s.nacc + (size_t)first * P + C * lane;
+#pragma unroll
+      for (int c = 0; c < C; c++)
+        if (acc.v[c] != kInf32) atomicMin(na + c, acc.v[c]);
       __threadfence();
       __syncwarp();
       uint32_t arrived = 0;
@@ -276,26 +290,18 @@ __global__ void __launch_bounds__(256, 3) mp32_iter_kernel(Mp32 s, uint32_t it) 
       arrived = __shfl_sync(0xffffffffu, arrived, 0);
       if (arrived == pieces - 1) {
         __threadfence();
-        uint32_t f = 0;
-        int4 nv = make_int4(0, 0, 0, 0);
-        if (sub == 0) {
-          const int4 got = make_int4(__ldcg(na), __ldcg(na + 1), __ldcg(na + 2), __ldcg(na + 3));
-          *reinterpret_cast<int4*>(na) = make_int4(kInf32, kInf32, kInf32, kInf32);
-          f = settle(row, got, nv);
+        Cols got;
+#pragma unroll
+        for (int c = 0; c < C; c++) {
+          got.v[c] = __ldcg(na + c);
+          na[c] = kInf32;
         }
-        if (__ballot_sync(0xffffffffu, f != 0)) {
-          if (sub == 0) *reinterpret_cast<int4*>(s.next + (size_t)row * P + c0) = nv;
-          if (lane == 0) atomicOr(fell_next + (row >> 5), 1u << (row & 31));
-        }
-        fell_cols |= f;
+        settle(row, got, x[(size_t)row * 32]);
         if (lane == 0) s.counters[first] = 0;
       }
     }
   }
-  // The columns that fell: lanes q of every group hold columns 4q..4q+3.
-#pragma unroll
-  for (uint32_t o = LPR; o < 32; o <<= 1) fell_cols |= __shfl_xor_sync(0xffffffffu, fell_cols, o);
-  if (sub == 0 && fell_cols) atomicOr(s.fell + (c0 >> 5), fell_cols << (c0 & 31));
+  if (fell_cols) atomicOr(s.fell + ((C * lane) >> 5), fell_cols << ((C * lane) & 31));
 }
 
 // Copies the rows that fell into the iterate; clears the bitmap the
@@ -398,20 +404,16 @@ wc_status mp32_pass(Ctx& ctx, const uint64_t* sources, const uint32_t* caps, con
   cudaStream_t st = ctx.stream;
   note_launch(), mp32_seed_kernel<P><<<max_blocks(4), 256, 0, st>>>(s, sources);
   note_launch(), mp32_sources_kernel<P><<<1, 128, 0, st>>>(s, sources);
-  const size_t smem = 8 * sizeof(Mp32Smem<P>);
-  static const cudaError_t attr = cudaFuncSetAttribute(
-      mp32_iter_kernel<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (attr != cudaSuccess) return cuda_status(attr, ctx.detail, "min-plus kernel attributes");
   const uint32_t grid = std::max<uint32_t>(1, std::min<uint32_t>(
-      max_blocks((int)blocks_per_sm), (csc.schedule.count + 7) / 8));
+      max_blocks((int)blocks_per_sm), (csc.schedule.count + kMp32Warps - 1) / kMp32Warps));
   const uint32_t apply_grid = std::max<uint32_t>(1, std::min<uint32_t>(
       max_blocks(8), (uint32_t)((words + 7) / 8)));
   for (uint32_t it = 0; it < max_cap; it++) {
-    note_launch(), mp32_iter_kernel<P><<<grid, 256, smem, st>>>(s, it);
+    note_launch(), mp32_iter_kernel<P><<<grid, 32 * kMp32Warps, 0, st>>>(s, it);
     note_launch(), mp32_apply_kernel<P><<<apply_grid, 256, 0, st>>>(s, it);
     note_launch(), mp32_control_kernel<P><<<1, 32, 0, st>>>(s, it);
   }
-  note_launch(), mp32_out_kernel<P><<<max_blocks(2), 256, 0, st>>>(s.x, n, k, cols, out);
+  note_launch(), mp32_out_kernel<P><<<max_blocks(8), 256, 0, st>>>(s.x, n, k, cols, out);
   return cuda_status(cudaGetLastError(), ctx.detail, "batched min-plus pass");
 }
 

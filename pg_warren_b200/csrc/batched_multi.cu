@@ -328,7 +328,7 @@ wc_status wc_minplus_batched(wc_version* v, const wc_call* call, const uint64_t*
       WC_TRY(ctx.run_captured(gk, [&] {
         return mp32_for(P32)(ctx, psrc_dev + c0, pcaps_dev + c0, pcols_dev + c0, k, max_cap,
                              static_cast<int64_t*>(D.dev), its->as<uint32_t>(),
-                             P32 == 64 ? 2 : 3);
+                             kMp32Blocks);
       }));
     }
     WC_TRY(D.out(ctx));
