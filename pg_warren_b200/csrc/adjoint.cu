@@ -46,35 +46,6 @@ struct AdjState {
   DeviceError* err;
 };
 
-template <int P> struct AdjEpi {
-  const AdjState* s;
-  int cur;
-  uint32_t run_bits;
-  double pi;  // this lane's column
-  double delta, total;
-  bool final_pass;
-  __device__ void cell(uint32_t i, uint32_t c, bool present, double z) {
-    const AdjState& st = *s;
-    const size_t at = (size_t)i * P + c;
-    const double o = st.out[i];
-    const double si = (present && o > 0.0) ? z / o : 0.0;
-    if (final_pass) {
-      st.S[at] = si;
-      return;
-    }
-    const double old = st.lam[cur][at];
-    if (!((run_bits >> c) & 1)) {
-      st.lam[cur ^ 1][at] = old;
-      total += old;
-      return;
-    }
-    const double next = st.damping * (si + (o > 0.0 ? 0.0 : pi)) + st.C[at];
-    delta += fabs(next - old);
-    total += next;
-    st.lam[cur ^ 1][at] = next;
-  }
-};
-
 template <int P>
 __global__ void adj_init_kernel(AdjState s) {
   double none = 0.0, total = 0.0;
@@ -95,36 +66,6 @@ __global__ void adj_init_kernel(AdjState s) {
     }
     if (threadIdx.x < s.k) s.iterations[threadIdx.x] = 0;
   }
-}
-
-template <int P, class W>
-__global__ void __launch_bounds__(256) adj_iter_kernel(CsrView<W> A, AdjState s, uint32_t it,
-                                                       Partial<double, WC_OP_PLUS>* carry,
-                                                       uint32_t max_iter) {
-  const uint32_t run = *(volatile uint32_t*)s.running;
-  if (!run) return;
-  const unsigned c = threadIdx.x % P;
-  AdjEpi<P> epi{&s, (int)(it & 1), run, s.pi[c], 0.0, 0.0, false};
-  pull_multi<double, WC_PLUS_TIMES, W, P>(A, s.lam[it & 1], epi, s.err, carry);
-  double delta = epi.delta, total = epi.total;
-  if (reduce_columns<P>(delta, total, s.partials, s.counter)) {
-    const uint32_t q = threadIdx.x;
-    if (q < P && ((run >> q) & 1)) {
-      s.pi[q] = s.p * total;
-      s.iterations[q] = it + 1;
-      if (it + 1 >= max_iter || delta < s.tol) atomicAnd(s.running, ~(1u << q));
-    }
-    if (q == 0) *s.executed = it + 1;
-  }
-}
-
-// S = D⁻¹ A λ for the final λ (the buffer the last iteration wrote).
-template <int P, class W>
-__global__ void __launch_bounds__(256) adj_rows_kernel(CsrView<W> A, AdjState s,
-                                                       Partial<double, WC_OP_PLUS>* carry) {
-  const int cur = *s.executed & 1;
-  AdjEpi<P> epi{&s, cur, 0, 0.0, 0.0, 0.0, true};
-  pull_multi<double, WC_PLUS_TIMES, W, P>(A, s.lam[cur], epi, s.err, carry);
 }
 
 // The same iteration and final pass over pull32_units (small blocks, as many
