@@ -48,7 +48,7 @@ __global__ void msbfs_seed_kernel(const uint64_t* sources, const uint32_t* caps,
                                   uint32_t levels, uint32_t n, uint32_t* V, uint32_t* F0,
                                   uint32_t* fbits0, uint32_t* wbits0, uint32_t* masks,
                                   uint32_t* alive0, uint32_t* counts, const uint32_t* foff,
-                                  unsigned long long* fedges0) {
+                                  unsigned long long* fedges0, const int32_t* cancel) {
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t < k) {
     const uint32_t node = (uint32_t)sources[t];
@@ -71,7 +71,9 @@ __global__ void msbfs_seed_kernel(const uint64_t* sources, const uint32_t* caps,
     }
     masks[x] = m;
   }
-  if (t == 0) counts[0] = 1;  // level 0's frontier is non-empty (or harmlessly so)
+  // Level 0's frontier is non-empty (or harmlessly so), unless the call is
+  // cancelled already.
+  if (t == 0) counts[0] = *(volatile const int32_t*)cancel ? 0u : 1u;
 }
 
 // Level L: F_{L+1}[i] = (OR over in-neighbours j in the frontier of
@@ -110,21 +112,27 @@ struct MsLevel {
   uint32_t* acc;      // n × W push accumulators, all zero between levels
   uint32_t* touched;  // rows with a push accumulator to settle, all zero between levels
   uint32_t* pulled;   // if set: counts the levels that pull (timed calls)
+  const int32_t* cancel;  // the caller's cancel word (host-mapped)
+  uint32_t* stopped;  // [level]: a cancel was raised before the level
   const uint32_t* unit_rows;  // per unit of `units`: its rows that hold entries
 };
 
-// Whether level P.L runs at all: it has a frontier.  A level that does not
-// run leaves the next level's count zero, so every later level returns at
-// once too.
-__device__ inline bool level_runs(const MsLevel& P) { return P.counts[P.L] != 0; }
+// Whether level P.L runs at all: it has a frontier, and no cancel was seen
+// before it.  A level that does not run leaves the next level's count zero,
+// so every later level returns at once too.
+__device__ inline bool level_runs(const MsLevel& P) {
+  return P.counts[P.L] != 0 && P.stopped[P.L] == 0;
+}
 
-// Before each level's kernels: a raised cancel word (host-mapped, read here
-// by one thread) empties the level's frontier count, so all of the level's
-// kernels and every later level return at once.  The count changes only
-// between kernels, so a level runs whole or not at all, and the buffers kept
-// zero between calls stay zero.
-__global__ void msbfs_cancel_kernel(const int32_t* cancel, uint32_t* count) {
-  if (threadIdx.x == 0 && *(volatile const int32_t*)cancel) *count = 0;
+// The caller's cancel word is read once a level that runs, by one thread of
+// its last kernel while that kernel's other blocks work, and stops the next
+// level.  A level's kernels all read what was there before its first, so a
+// level runs whole or not at all, and the buffers kept zero between calls stay
+// zero.  (A kernel of its own a level cost a batch of 100 searches over
+// 150,001 nodes 16 launches, 25 of 427 µs.)
+__device__ inline void read_cancel(const MsLevel& P) {
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0 && *(volatile const int32_t*)P.cancel)
+    P.stopped[P.L + 1] = 1;
 }
 
 // A level pushes (scatters the frontier rows over the forward CSR) while the
@@ -230,6 +238,7 @@ __device__ inline void prefetch_unit(const MsLevel& P, const Unit& d, uint32_t h
 template <int W>
 __global__ void __launch_bounds__(256, 4) msbfs_level_kernel(MsLevel P) {
   if (!level_runs(P)) return;  // nothing expands (or cancelled): F_{L+1} is not read
+  read_cancel(P);
   if (level_pushes(P)) return;  // msbfs_push_kernel and msbfs_settle_kernel run it
   if (P.pulled && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(P.pulled, 1u);
   constexpr uint32_t VEC = W >= 4 ? 4 : W;
@@ -990,6 +999,29 @@ __global__ void __launch_bounds__(kDepthBlock, 1)
       const uint32_t node = i0 + 16 * p;
       const bool whole = aligned16 && node + 16 <= n;
       uint8_t* dst = depth_out + (size_t)(4 * g) * n + node;
+      if (!aligned16 && i0 + TN <= n) {
+        // Rows that start anywhere: the run of 64 bytes shifted to the words
+        // of memory it covers, whole words but at its two ends, which are
+        // other tiles' too.  (A byte a store, 100 sources over 150,001 nodes
+        // took 97 of 427 µs.)
+#pragma unroll
+        for (uint32_t t4 = 0; t4 < 4; t4++, dst += n) {
+          const uint32_t before = __shfl_up_sync(0xffffffffu, o[3][t4], 1);
+          if (4 * g + t4 >= k) continue;
+          const uint32_t a = (uint32_t)(reinterpret_cast<uintptr_t>(dst) & 3u), sh = 8 * a;
+          uint32_t* words = reinterpret_cast<uint32_t*>(dst - a);
+          if (a == 0 || p != 0) words[0] = __funnelshift_l(before, o[0][t4], sh);
+          else
+            for (uint32_t r = 0; r < 4 - a; r++) dst[r] = (uint8_t)(o[0][t4] >> (8 * r));
+          words[1] = __funnelshift_l(o[0][t4], o[1][t4], sh);
+          words[2] = __funnelshift_l(o[1][t4], o[2][t4], sh);
+          words[3] = __funnelshift_l(o[2][t4], o[3][t4], sh);
+          if (p == 3)
+            for (uint32_t r = 4 - a; r < 4; r++)
+              dst[12 + r] = (uint8_t)(o[3][t4] >> (8 * r));
+        }
+        continue;
+      }
 #pragma unroll
       for (uint32_t t4 = 0; t4 < 4; t4++, dst += n) {
         if (4 * g + t4 >= k) break;
@@ -1124,7 +1156,7 @@ wc_status run_pass(Ctx& ctx, BatchBuffers& b, const uint64_t* sources_dev, const
   note_launch(), msbfs_clear_kernel<W><<<(k + 255) / 256, 256, 0, st>>>(sources_dev, k, F);
   note_launch(), msbfs_seed_kernel<W><<<std::max<uint32_t>(1, (std::max(k, (levels + 1) * W) + 255) / 256), 256, 0,
                          st>>>(sources_dev, caps_dev, k, levels + 1, n, V, F, fbits, wbits, masks,
-                               alive, counts, foff, fedges);
+                               alive, counts, foff, fedges, v->cancel_dev);
   const DevCsr& csc = v->rev;
   const size_t level_smem = 8 * sizeof(MsWarpSmem<W>);
   if (level_smem > 48 * 1024)
@@ -1147,9 +1179,8 @@ wc_status run_pass(Ctx& ctx, BatchBuffers& b, const uint64_t* sources_dev, const
               fbits + (L + 1) * bitmap_words, wbits + (L + 1) * bitmap_words, masks, alive, L,
               counts, fedges, foff, fwd.targets.as<uint32_t>(), fwd.schedule.units.as<Unit>(),
               fwd.schedule.count, v->m, b.acc->as<uint32_t>(), b.touched->as<uint32_t>(),
-              b.pulled ? b.pulled->as<uint32_t>() : nullptr,
+              b.pulled ? b.pulled->as<uint32_t>() : nullptr, v->cancel_dev, counts + (levels + 2),
               csc.schedule.row_masks.as<uint32_t>()};
-    note_launch(), msbfs_cancel_kernel<<<1, 32, 0, st>>>(v->cancel_dev, counts + L);
     note_launch(), msbfs_push_kernel<W><<<push_grid, 256, 0, st>>>(P);
     note_launch(), msbfs_settle_kernel<W><<<settle_grid, 256, 0, st>>>(P);
     // The pull alone is timed too ("pull"), for its roofline.
