@@ -1173,14 +1173,14 @@ wc_status run_pass(Ctx& ctx, BatchBuffers& b, const uint64_t* sources_dev, const
   // that the level's frontier does not call for return at once.
   ctx.phase_begin("level");
   for (uint32_t L = 0; L < levels; L++) {
-    MsLevel P{n, csc.offsets.as<uint32_t>(), csc.targets.as<uint32_t>(), csc.schedule.units.as<Unit>(),
+    MsLevel P{n, csc.offsets.as<uint32_t>(), csc.targets.as<uint32_t>(), csc.schedule.rounds.as<Unit>(),
               csc.schedule.count, csc.schedule.counters.as<uint32_t>(), b.nacc->as<uint32_t>(), V,
               F + L * fstride, F + (L + 1) * fstride, fbits + L * bitmap_words,
               fbits + (L + 1) * bitmap_words, wbits + (L + 1) * bitmap_words, masks, alive, L,
               counts, fedges, foff, fwd.targets.as<uint32_t>(), fwd.schedule.units.as<Unit>(),
               fwd.schedule.count, v->m, b.acc->as<uint32_t>(), b.touched->as<uint32_t>(),
               b.pulled ? b.pulled->as<uint32_t>() : nullptr, v->cancel_dev, counts + (levels + 2),
-              csc.schedule.row_masks.as<uint32_t>()};
+              csc.schedule.round_masks.as<uint32_t>()};
     note_launch(), msbfs_push_kernel<W><<<push_grid, 256, 0, st>>>(P);
     note_launch(), msbfs_settle_kernel<W><<<settle_grid, 256, 0, st>>>(P);
     // The pull alone is timed too ("pull"), for its roofline.

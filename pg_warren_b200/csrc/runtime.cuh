@@ -236,7 +236,12 @@ struct Schedule {
   DevBuf counters;    // u32[slots]: arrivals per long row (indexed by its first slot)
   DevBuf carry;       // the pieces' partial results, kCarryBytesPerSlot per slot
   DevBuf long_list;   // uint4[long_rows]: each long row, its first slot and piece count
-  DevBuf row_masks;   // u32[count]: a tile's rows that hold entries (bit r: row a + r)
+  // The reverse CSR's units again, for the batched BFS (count of them): the
+  // long rows' first pieces, the tiles, then the other pieces by their place
+  // in their row, so that a row's later pieces come after its earlier ones
+  // have left their bits.  round_masks: per unit, a tile's rows that hold
+  // entries (bit r: row a + r).
+  DevBuf rounds, round_masks;
   uint32_t count = 0;
   uint32_t slots = 0;
   uint32_t long_rows = 0;
@@ -263,7 +268,7 @@ struct LaneCsr {
   DevBuf rows, lengths;      // u32 / u16: row ids sorted by length, longest first; their entries
   DevBuf targets, weights, iweights;
   DevBuf hot;                // u32[hot_count]: the hot nodes, most gathered first
-  uint32_t count = 0;
+  uint32_t count = 0, groups = 0;  // units; of which (the first) of long rows
   uint32_t filled = 0, shorts = 0;  // of `rows`: those with entries, then to here the empty ones
   uint32_t hot_count = 0;
   uint32_t run = 1;     // pieces of a long row a unit takes at most

@@ -17,7 +17,7 @@ wc_status device_reverse(wc_version* v, wc_error_detail* detail);
 // Every target of the forward CSR against the id space, on the device: the
 // first outside it is WC_NODE_OUTSIDE_ID_SPACE with the target in the detail.
 wc_status device_targets_in_space(wc_version* v, wc_error_detail* detail);
-// The schedule's per-unit masks of the rows that hold entries.
+// The masks of the batched BFS's units (Schedule::round_masks).
 wc_status device_row_masks(wc_version* v, DevCsr& d, wc_error_detail* detail);
 // Whether every weight is an i32 integer (then i32 copies of both
 // orientations' weights) and the largest magnitude.

@@ -88,6 +88,32 @@ static wc_status put_csr(wc_version* v, DevCsr& d, const uint64_t* off, const ui
   return cuda_status(cudaStreamSynchronize(v->stream), detail, "version upload");
 }
 
+// The units in the batched BFS's order (Schedule::rounds), by a counting sort.
+static wc_status put_rounds(wc_version* v, DevCsr& d, const std::vector<Unit>& units,
+                            const std::vector<uint64_t>& off, wc_error_detail* detail) {
+  Schedule& s = d.schedule;
+  auto round_of = [&](const Unit& u) -> uint32_t {
+    if ((u.c >> 31) == 0) return 1;
+    const uint32_t p = (uint32_t)((u.b - off[u.a]) / kPieceEntries);
+    return p == 0 ? 0 : p + 1;
+  };
+  std::vector<uint32_t> first(3, 0);
+  for (const Unit& u : units) {
+    const uint32_t q = round_of(u) + 1;
+    if (q >= first.size()) first.resize(q + 1, 0);
+    first[q]++;
+  }
+  for (size_t q = 1; q < first.size(); q++) first[q] += first[q - 1];
+  std::vector<Unit> ordered(units.size());
+  for (const Unit& u : units) ordered[first[round_of(u)]++] = u;
+  WC_TRY(s.rounds.alloc(v->budget, std::max<size_t>(units.size(), 1) * sizeof(Unit), detail));
+  if (!units.empty())
+    WC_CUDA(cudaMemcpy(s.rounds.ptr, ordered.data(), ordered.size() * sizeof(Unit),
+                       cudaMemcpyHostToDevice), detail);
+  WC_TRY(s.round_masks.alloc(v->budget, std::max<size_t>(units.size(), 1) * 4, detail));
+  return device_row_masks(v, d, detail);
+}
+
 // The schedule of one orientation from its host offsets.
 wc_status put_schedule(wc_version* v, DevCsr& d, const std::vector<uint64_t>& off,
                               wc_error_detail* detail) {
@@ -118,9 +144,7 @@ wc_status put_schedule(wc_version* v, DevCsr& d, const std::vector<uint64_t>& of
   if (!longs.empty())
     WC_CUDA(cudaMemcpy(s.long_list.ptr, longs.data(), longs.size() * 4, cudaMemcpyHostToDevice),
             detail);
-  // Per tile, its rows that hold entries (a piece's row always does).
-  WC_TRY(s.row_masks.alloc(v->budget, std::max<size_t>(units.size(), 1) * 4, detail));
-  return device_row_masks(v, d, detail);
+  return &d == &v->rev ? put_rounds(v, d, units, off, detail) : WC_OK;
 }
 
 wc_status wc_device_check(wc_error_detail* detail) {
@@ -301,7 +325,8 @@ wc_status wc_version_info_get(const wc_version* v, wc_version_info* info) {
   for (const DevCsr* d : {&v->fwd, &v->rev, &v->loc.csc})
     bytes += d->offsets.bytes + d->targets.bytes + d->weights.bytes + d->iweights.bytes +
              d->schedule.units.bytes + d->schedule.counters.bytes + d->schedule.carry.bytes +
-             d->schedule.long_list.bytes + d->schedule.row_masks.bytes + d->lanes.bytes();
+             d->schedule.long_list.bytes + d->schedule.rounds.bytes + d->schedule.round_masks.bytes +
+             d->lanes.bytes();
   bytes += v->loc.perm.bytes + v->loc.order.bytes + v->loc.lane_targets.bytes +
            v->loc.lane_hot.bytes;
   info->device_bytes = bytes;
