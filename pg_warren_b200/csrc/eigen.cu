@@ -69,13 +69,17 @@ __global__ void sum_partial_kernel(uint32_t n, F f, double* partial) {
 // order by one thread from there, so the dependent chain of additions waits
 // on shared memory rather than on L2.
 constexpr uint32_t kSumFinalMaxValues = kRedBlocks * 8;  // count × columns
+// `host` (mapped memory, may be NULL) gets the sums too: a copy queued behind
+// each of a step's reductions cost the host as much again as its wait.
 __global__ void __launch_bounds__(256) sum_final_kernel(const double* partial, uint32_t count,
-                                                        uint32_t columns, double* out) {
+                                                        uint32_t columns, double* out,
+                                                        double* host) {
   __shared__ double sp[kSumFinalMaxValues];
   // Block b combines the b-th run of count × columns partials into
   // out[b·columns ..): several projections' partials in one launch.
   partial += (size_t)blockIdx.x * count * columns;
   out += (size_t)blockIdx.x * columns;
+  if (host) host += (size_t)blockIdx.x * columns;
   const uint32_t total = count * columns;
   for (uint32_t i = threadIdx.x; i < total; i += blockDim.x) sp[i] = partial[i];
   __syncthreads();
@@ -83,6 +87,7 @@ __global__ void __launch_bounds__(256) sum_final_kernel(const double* partial, u
     double t = 0.0;
     for (uint32_t b = 0; b < count; b++) t += sp[b * columns + c];
     out[c] = t;
+    if (host) *(volatile double*)(host + c) = t;
   }
 }
 
@@ -422,6 +427,17 @@ __global__ void scale_vec_kernel(double* x, uint32_t n, double f) {
     x[i] *= f;
 }
 
+// A new basis vector q = w · f and, for the normalised operators, its scaled
+// copy that the next product reads (scale_kernel's), in one pass.
+__global__ void push_kernel(const double* w, uint32_t n, double f, double* q, const double* scale,
+                            double* scaled) {
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const double x = w[i] * f;
+    q[i] = x;
+    if (scale) scaled[i] = scale[i] * x;
+  }
+}
+
 __global__ void residual_terms_kernel(const double* x, const double* y, double value, uint32_t n,
                                       double* partial) {
   __shared__ double s[32];
@@ -562,11 +578,11 @@ struct Eigensolver {
 
   wc_status sum_final(uint32_t count, uint32_t columns, double* out_host) {
     if ((uint64_t)count * columns > kSumFinalMaxValues) return WC_INVALID_ARGUMENT;
-    note_launch(), sum_final_kernel<<<1, 256, 0, st()>>>(partial->as<double>(), count, columns,
-                                                         coefbuf->as<double>());
-    WC_CUDA(cudaMemcpyAsync(out_host, coefbuf->ptr, columns * 8, cudaMemcpyDeviceToHost, st()),
-            ctx.detail);
+    note_launch(), sum_final_kernel<<<1, 256, 0, st()>>>(
+        partial->as<double>(), count, columns, coefbuf->as<double>(),
+        reinterpret_cast<double*>(v->stage_dev + kStagePlan));
     WC_CUDA(cudaStreamSynchronize(st()), ctx.detail);
+    std::memcpy(out_host, v->stage_host + kStagePlan, columns * 8);
     return WC_OK;
   }
 
@@ -594,8 +610,10 @@ struct Eigensolver {
   wc_status apply(const double* x, double* out) {
     const double* src = x;
     if (normalized) {
-      note_launch(), scale_kernel<<<grid, 256, 0, st()>>>(x, scale->as<double>(), scaled->as<double>(), n);
+      if (x != scaled_of)
+        note_launch(), scale_kernel<<<grid, 256, 0, st()>>>(x, scale->as<double>(), scaled->as<double>(), n);
       src = scaled->as<double>();
+      scaled_of = nullptr;
     }
     WC_TRY(multiply(src, out, o.weighted));
     note_launch(), finish_apply_kernel<<<grid, 256, 0, st()>>>(op, x, out);
@@ -792,6 +810,9 @@ struct Eigensolver {
 
   // ---------------------------------------------------------- the basis
   uint32_t size = 0, len = 0;
+  // The basis vector whose scaled copy the last push left in `scaled`, until
+  // it is applied.
+  const double* scaled_of = nullptr;
   uint32_t held_chunks = 1;  // projection chunks the partial and coefficient buffers hold
 
   double* col(uint32_t j) { return Q->as<double>() + (size_t)j * n; }
@@ -815,12 +836,9 @@ struct Eigensolver {
                                                             pending, c,
                                                             partial->as<double>() +
                                                                 (size_t)b * grid * 8);
-    note_launch(), sum_final_kernel<<<chunks, 256, 0, st()>>>(partial->as<double>(), grid, 8,
-                                                              coefbuf->as<double>());
-    if (len)
-      WC_CUDA(cudaMemcpyAsync(v->stage_host + kStagePayload, coefbuf->ptr, len * 8,
-                              cudaMemcpyDeviceToHost, st()),
-              ctx.detail);
+    note_launch(), sum_final_kernel<<<chunks, 256, 0, st()>>>(
+        partial->as<double>(), grid, 8, coefbuf->as<double>(),
+        reinterpret_cast<double*>(v->stage_dev + kStagePayload));
     return WC_OK;
   }
 
@@ -869,8 +887,10 @@ struct Eigensolver {
 
   wc_status push(const double* w, double norm) {
     if (len == size) return WC_OK;
-    note_launch(), copy_kernel<<<grid, 256, 0, st()>>>(w, col(len), n);
-    note_launch(), scale_vec_kernel<<<grid, 256, 0, st()>>>(col(len), n, 1.0 / norm);
+    note_launch(), push_kernel<<<grid, 256, 0, st()>>>(
+        w, n, 1.0 / norm, col(len), normalized ? scale->as<double>() : nullptr,
+        scaled->as<double>());
+    scaled_of = normalized ? col(len) : nullptr;
     len++;
     return cuda_status(cudaGetLastError(), ctx.detail, "push");
   }
