@@ -381,7 +381,7 @@ def _spmv_sweep(W, O, torch, dev, stream, peak, g, cpu):
 
 def spmv_point(W, torch, dev, stream, peak, g):
     """plus_times f64 over the reverse CSR (pull, the reference's transpose
-    product), R-MAT 22, 20 iterations from a 1% vector: spmv_pull_kernel's
+    product), R-MAT 22, 20 iterations from a 1% vector: spmv_lane_kernel's
     fraction of the roofline, bytes 4(n+1) + 12m + 16n an iteration."""
     n, m = g.id_space, g.edges
     rng = np.random.default_rng(SEED)
@@ -404,7 +404,7 @@ def spmv_point(W, torch, dev, stream, peak, g):
     ms = a.elapsed_time(b) / 20
     bytes_it = 4 * (n + 1) + 12 * m + 16 * n
     gbs = bytes_it / (ms * 1e-3) / 1e9
-    return {"kernel": "spmv_pull_kernel", "semiring": "plus_times", "dtype": "f64",
+    return {"kernel": "spmv_lane_kernel", "semiring": "plus_times", "dtype": "f64",
             "us_per_iteration": ms * 1e3, "bytes_per_iteration": bytes_it,
             "achieved": gbs, "peak": peak, "unit": "GB/s", "frac": gbs / peak}
 
@@ -1090,7 +1090,7 @@ def main():
     pr_kernel_gbs = pr_bytes * pr_it * args.steps / (pr_iter_ms * 1e-3) / 1e9 if pr_iter_ms else 0.0
     pagerank = {"iterations": pr_it, "ms": statistics.median(pr_ms),
                 "iters_per_s": pr_it / (statistics.median(pr_ms) * 1e-3),
-                "roofline": {"bound": "hbm", "kernel": "pr_iter_kernel",
+                "roofline": {"bound": "hbm", "kernel": "pr_lane_kernel",
                              "achieved": pr_kernel_gbs, "peak": peak, "unit": "GB/s",
                              "frac": pr_kernel_gbs / peak,
                              "bytes_per_iteration": pr_bytes}}
