@@ -33,6 +33,7 @@ struct Mp32 {
   const int32_t* w;    // NULL: unweighted (every weight 1)
   const Unit* units;
   uint32_t unit_count;
+  uint32_t split;      // warps a tile's rows are dealt to
   uint32_t* counters;  // per long row (first slot), left zero
   int32_t* nacc;       // P per long row (first slot), left at kInf32
   int32_t* x;          // n × P: the current iterate
@@ -165,12 +166,28 @@ __global__ void __launch_bounds__(32 * kMp32Warps, 5) mp32_iter_kernel(Mp32 s, u
     fell_cols |= f;
   };
 
+  // Part `u % split` of unit u / split: of a tile the part's share of its
+  // rows, of a piece all of it in the first part.
+  const uint32_t parts = s.unit_count * s.split;
+  auto part_of = [&](uint32_t u) {
+    Unit d = s.units[u / s.split];
+    const uint32_t part = u % s.split;
+    if (s.split == 1) return d;
+    if (d.c >> 31) {
+      if (part) d = Unit{d.a, d.a, 0u, 0u};  // an empty tile
+      return d;
+    }
+    const uint32_t rows = d.b - d.a;
+    const uint32_t a = d.a + rows * part / s.split, b = d.a + rows * (part + 1) / s.split;
+    const uint32_t lo = __ldg(s.off + a);
+    return Unit{a, b, __ldg(s.off + b) - lo, lo};
+  };
   Unit ahead{};
-  if (warp < s.unit_count) ahead = s.units[warp];
-  for (uint32_t u = warp; u < s.unit_count; u += warps) {
+  if (warp < parts) ahead = part_of(warp);
+  for (uint32_t u = warp; u < parts; u += warps) {
     const Unit unit = ahead;
-    if (u + warps < s.unit_count) {
-      ahead = s.units[u + warps];
+    if (u + warps < parts) {
+      ahead = part_of(u + warps);
       if (32 * lane < unit_count(ahead))  // its targets into L2 meanwhile
         asm volatile("prefetch.global.L2 [%0];" ::"l"(s.tgt + unit_first(ahead) + 32 * lane));
     }
@@ -404,8 +421,15 @@ wc_status mp32_pass(Ctx& ctx, const uint64_t* sources, const uint32_t* caps, con
   cudaStream_t st = ctx.stream;
   note_launch(), mp32_seed_kernel<P><<<max_blocks(4), 256, 0, st>>>(s, sources);
   note_launch(), mp32_sources_kernel<P><<<1, 128, 0, st>>>(s, sources);
-  const uint32_t grid = std::max<uint32_t>(1, std::min<uint32_t>(
-      max_blocks((int)blocks_per_sm), (csc.schedule.count + kMp32Warps - 1) / kMp32Warps));
+  // A graph of fewer units than the chip holds warps has each tile's rows dealt
+  // to up to four (a warp's sixteen batches of a whole tile are what such an
+  // iteration waits for: 71 searches over 17,533 nodes, 1.29 ms undealt).
+  s.split = std::max<uint32_t>(
+      1, std::min<uint32_t>(4, max_blocks((int)blocks_per_sm) * kMp32Warps /
+                                   std::max<uint32_t>(1, csc.schedule.count)));
+  const uint64_t parts = (uint64_t)csc.schedule.count * s.split;
+  const uint32_t grid = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(
+      max_blocks((int)blocks_per_sm), (parts + kMp32Warps - 1) / kMp32Warps));
   const uint32_t apply_grid = std::max<uint32_t>(1, std::min<uint32_t>(
       max_blocks(8), (uint32_t)((words + 7) / 8)));
   for (uint32_t it = 0; it < max_cap; it++) {
