@@ -7,7 +7,8 @@
 // plus) maps to i32::MAX: the distances and the per-column iteration counts
 // are the i64 loop's.
 //
-// A pass runs P = 32 or 64 columns, P / 32 a lane.  An iteration reads
+// A pass runs P = 32 or 64 columns: two a lane in the row kernel (64), four a
+// lane in the tile kernel (mp32_rows says which).  An iteration reads
 // the previous iterate only (next = min(x, Aᵀ ⊗ x)); after iteration t every
 // row holds x_i ≤ x_j + w for the values of iteration t-1, so iteration t+1
 // folds only the entries whose source row fell at t (a bitmap).  Rows that
@@ -33,7 +34,6 @@ struct Mp32 {
   const int32_t* w;    // NULL: unweighted (every weight 1)
   const Unit* units;
   uint32_t unit_count;
-  uint32_t split;      // warps a tile's rows are dealt to
   uint32_t* counters;  // per long row (first slot), left zero
   int32_t* nacc;       // P per long row (first slot), left at kInf32
   int32_t* x;          // n × P: the current iterate
@@ -56,9 +56,6 @@ constexpr uint32_t kMp32Unroll = 16;  // entries gathered at once
 // A lane's columns of a row.
 template <int C> struct alignas(4 * C) Cols32 { int32_t v[C]; };
 
-__device__ inline Cols32<1> load_cols(const Cols32<1>* p) {
-  return Cols32<1>{{__ldg(p->v)}};
-}
 __device__ inline Cols32<2> load_cols(const Cols32<2>* p) {
   const int2 v = __ldg(reinterpret_cast<const int2*>(p));
   return Cols32<2>{{v.x, v.y}};
@@ -108,6 +105,220 @@ __global__ void mp32_sources_kernel(Mp32 s, const uint64_t* sources) {
     s.x[(size_t)node * P + c] = 0;
     atomicOr(s.fell_rows[0] + (node >> 5), 1u << (node & 31));
   }
+}
+
+template <int P> struct Mp32Smem {
+  int32_t acc[32 * P];
+  uint32_t hitj[kTileEntries];
+  int32_t hitw[kTileEntries];
+  uint8_t hitr[kTileEntries];
+  uint8_t rowof[kTileEntries];
+};
+
+// One iteration over the reverse CSR's schedule: the rows' minima in shared
+// memory, a row's P distances spread over P/4 lanes.  What the passes run that
+// mp32_iter_kernel does not suit (mp32_rows below): a tile costs it the same
+// whatever number of its rows had hits.
+template <int P>
+__global__ void __launch_bounds__(256, 3) mp32_tile_kernel(Mp32 s, uint32_t it) {
+  constexpr uint32_t LPR = P / 4;       // lanes a row
+  constexpr uint32_t G = 32 / LPR;      // rows (or gathered rows) a warp instruction covers
+  constexpr uint32_t GM = LPR == 32 ? 0xffffffffu : (1u << LPR) - 1;
+  constexpr int Q = kTileEntries / 32;
+  constexpr int U = 8;
+  constexpr uint32_t VR = kTileRows / G;
+  bool any_running = false;
+  for (uint32_t q = 0; q < P / 32; q++) any_running |= s.running[q] != 0;
+  if (!any_running) return;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  Mp32Smem<P>& sm = reinterpret_cast<Mp32Smem<P>*>(smem_raw)[threadIdx.x >> 5];
+  const unsigned lane = threadIdx.x & 31;
+  const unsigned sub = lane / LPR, q = lane % LPR;
+  const uint32_t c0 = q * 4;  // this lane's four columns
+  const unsigned gmask = GM << (sub * LPR);
+  const uint32_t run4 = (s.running[c0 >> 5] >> (c0 & 31)) & 0xFu;  // running bits of c0..c0+3
+  const uint32_t* fell_cur = s.fell_rows[it & 1];
+  uint32_t* fell_next = s.fell_rows[(it + 1) & 1];
+  const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+  uint32_t fell_cols = 0;  // bits of this lane's four columns that fell
+
+  // new = min(old, got) for running columns; f: the columns that fell.
+  auto settle = [&](uint32_t i, const int4& got, int4& nv) -> uint32_t {
+    const int4 old = *reinterpret_cast<const int4*>(s.x + (size_t)i * P + c0);
+    nv = old;
+    if ((run4 & 1) && got.x < old.x) nv.x = got.x;
+    if ((run4 & 2) && got.y < old.y) nv.y = got.y;
+    if ((run4 & 4) && got.z < old.z) nv.z = got.z;
+    if ((run4 & 8) && got.w < old.w) nv.w = got.w;
+    return (nv.x < old.x ? 1u : 0u) | (nv.y < old.y ? 2u : 0u) | (nv.z < old.z ? 4u : 0u) |
+           (nv.w < old.w ? 8u : 0u);
+  };
+
+  for (uint32_t u = warp; u < s.unit_count; u += warps) {
+    const Unit unit = s.units[u];
+    const bool tile = (unit.c >> 31) == 0;
+    const uint32_t r0 = unit.a;
+    const uint32_t R = tile ? unit.b - unit.a : 1;
+    uint32_t base, count;
+    if (tile) {
+      uint32_t lo = 0, hi = 0;
+      if (lane < R) {
+        lo = __ldg(s.off + r0 + lane);
+        hi = __ldg(s.off + r0 + lane + 1);
+      }
+      base = unit.d;
+      count = unit.c;
+      for (uint32_t k = lo - base; k < hi - base; k++) sm.rowof[k] = (uint8_t)lane;
+      for (uint32_t x = lane * 4; x < R * P; x += 128)
+        *reinterpret_cast<int4*>(&sm.acc[x]) = make_int4(kInf32, kInf32, kInf32, kInf32);
+    } else {
+      base = unit.b;
+      count = unit.d - unit.b;
+    }
+    __syncwarp();
+    // The hits: entries whose source row fell in the previous iteration.
+    uint32_t H = 0;
+    {
+      uint32_t jv[Q];
+#pragma unroll
+      for (int qq = 0; qq < Q; qq++) {
+        const uint32_t k = lane + 32 * qq;
+        jv[qq] = k < count ? __ldcs(s.tgt + base + k) : 0u;
+      }
+#pragma unroll
+      for (int qq = 0; qq < Q; qq++) {
+        const uint32_t k = lane + 32 * qq;
+        const bool hit = k < count && ((fell_cur[jv[qq] >> 5] >> (jv[qq] & 31)) & 1);
+        const uint32_t m = __ballot_sync(0xffffffffu, hit);
+        if (hit) {
+          const uint32_t pos = H + __popc(m & ((1u << lane) - 1));
+          sm.hitj[pos] = jv[qq];
+          sm.hitw[pos] = s.w ? __ldg(s.w + base + k) : 1;
+          sm.hitr[pos] = tile ? sm.rowof[k] : (uint8_t)0;
+        }
+        H += __popc(m);
+      }
+    }
+    __syncwarp();
+    // Gather: group g takes hits [g·H/G, (g+1)·H/G) in order; a row's hits
+    // are consecutive, so their minima stay in registers until the row
+    // changes.
+    int4 run = make_int4(kInf32, kInf32, kInf32, kInf32);
+    if (H) {
+      const uint32_t per = (H + G - 1) / G;
+      const uint32_t h_lo = min(H, sub * per), h_hi = min(H, sub * per + per);
+      uint32_t cur = h_lo < h_hi ? sm.hitr[h_lo] : 0u;
+      for (uint32_t h0 = h_lo; h0 < h_hi; h0 += U) {
+        int4 val[U];
+        int32_t wv[U];
+        uint32_t rr[U];
+#pragma unroll
+        for (int x = 0; x < U; x++) {
+          const uint32_t h = h0 + x;
+          rr[x] = cur;
+          wv[x] = 0;
+          val[x] = make_int4(kInf32, kInf32, kInf32, kInf32);
+          if (h < h_hi) {
+            val[x] = __ldg(reinterpret_cast<const int4*>(s.x + (size_t)sm.hitj[h] * P + c0));
+            wv[x] = sm.hitw[h];
+            rr[x] = sm.hitr[h];
+          }
+        }
+#pragma unroll
+        for (int x = 0; x < U; x++) {
+          if (rr[x] != cur) {
+            if (tile) {
+              int32_t* a = &sm.acc[cur * P + c0];
+              if (run.x != kInf32) atomicMin(a, run.x);
+              if (run.y != kInf32) atomicMin(a + 1, run.y);
+              if (run.z != kInf32) atomicMin(a + 2, run.z);
+              if (run.w != kInf32) atomicMin(a + 3, run.w);
+            }
+            run = make_int4(kInf32, kInf32, kInf32, kInf32);
+            cur = rr[x];
+          }
+          run.x = min(run.x, add_absorbing(val[x].x, wv[x]));
+          run.y = min(run.y, add_absorbing(val[x].y, wv[x]));
+          run.z = min(run.z, add_absorbing(val[x].z, wv[x]));
+          run.w = min(run.w, add_absorbing(val[x].w, wv[x]));
+        }
+      }
+      if (tile) {
+        int32_t* a = &sm.acc[cur * P + c0];
+        if (run.x != kInf32) atomicMin(a, run.x);
+        if (run.y != kInf32) atomicMin(a + 1, run.y);
+        if (run.z != kInf32) atomicMin(a + 2, run.z);
+        if (run.w != kInf32) atomicMin(a + 3, run.w);
+      }
+    }
+    __syncwarp();
+    if (tile) {
+#pragma unroll
+      for (uint32_t x = 0; x < VR; x++) {
+        if (x * G >= R) break;
+        const uint32_t r = x * G + sub;
+        uint32_t f = 0;
+        int4 nv = make_int4(0, 0, 0, 0);
+        if (r < R) {
+          const int4 got = *reinterpret_cast<const int4*>(&sm.acc[r * P + c0]);
+          f = settle(r0 + r, got, nv);
+        }
+        if (__ballot_sync(0xffffffffu, f != 0) & gmask) {
+          *reinterpret_cast<int4*>(s.next + (size_t)(r0 + r) * P + c0) = nv;
+          if (q == 0) atomicOr(fell_next + ((r0 + r) >> 5), 1u << ((r0 + r) & 31));
+        }
+        fell_cols |= f;
+      }
+      __syncwarp();
+    } else {
+      // The groups' minima, then into the row's global accumulator.
+#pragma unroll
+      for (uint32_t o = LPR; o < 32; o <<= 1) {
+        run.x = min(run.x, __shfl_xor_sync(0xffffffffu, run.x, o));
+        run.y = min(run.y, __shfl_xor_sync(0xffffffffu, run.y, o));
+        run.z = min(run.z, __shfl_xor_sync(0xffffffffu, run.z, o));
+        run.w = min(run.w, __shfl_xor_sync(0xffffffffu, run.w, o));
+      }
+      const uint32_t row = unit.a, slot = unit.c & 0x7fffffffu;
+      const uint32_t row_lo = __ldg(s.off + row);
+      const uint32_t deg = __ldg(s.off + row + 1) - row_lo;
+      const uint32_t pieces = (deg + kPieceEntries - 1) / kPieceEntries;
+      const uint32_t first = slot - (unit.b - row_lo) / kPieceEntries;
+      int32_t* na = s.nacc + (size_t)first * P + c0;
+      if (sub == 0) {
+        if (run.x != kInf32) atomicMin(na, run.x);
+        if (run.y != kInf32) atomicMin(na + 1, run.y);
+        if (run.z != kInf32) atomicMin(na + 2, run.z);
+        if (run.w != kInf32) atomicMin(na + 3, run.w);
+      }
+      __threadfence();
+      __syncwarp();
+      uint32_t arrived = 0;
+      if (lane == 0) arrived = atomicAdd(s.counters + first, 1u);
+      arrived = __shfl_sync(0xffffffffu, arrived, 0);
+      if (arrived == pieces - 1) {
+        __threadfence();
+        uint32_t f = 0;
+        int4 nv = make_int4(0, 0, 0, 0);
+        if (sub == 0) {
+          const int4 got = make_int4(__ldcg(na), __ldcg(na + 1), __ldcg(na + 2), __ldcg(na + 3));
+          *reinterpret_cast<int4*>(na) = make_int4(kInf32, kInf32, kInf32, kInf32);
+          f = settle(row, got, nv);
+        }
+        if (__ballot_sync(0xffffffffu, f != 0)) {
+          if (sub == 0) *reinterpret_cast<int4*>(s.next + (size_t)row * P + c0) = nv;
+          if (lane == 0) atomicOr(fell_next + (row >> 5), 1u << (row & 31));
+        }
+        fell_cols |= f;
+        if (lane == 0) s.counters[first] = 0;
+      }
+    }
+  }
+  // The columns that fell: lanes q of every group hold columns 4q..4q+3.
+#pragma unroll
+  for (uint32_t o = LPR; o < 32; o <<= 1) fell_cols |= __shfl_xor_sync(0xffffffffu, fell_cols, o);
+  if (sub == 0 && fell_cols) atomicOr(s.fell + (c0 >> 5), fell_cols << (c0 & 31));
 }
 
 // One iteration over the reverse CSR's schedule: a warp per unit, a row of x
@@ -166,28 +377,12 @@ __global__ void __launch_bounds__(32 * kMp32Warps, 5) mp32_iter_kernel(Mp32 s, u
     fell_cols |= f;
   };
 
-  // Part `u % split` of unit u / split: of a tile the part's share of its
-  // rows, of a piece all of it in the first part.
-  const uint32_t parts = s.unit_count * s.split;
-  auto part_of = [&](uint32_t u) {
-    Unit d = s.units[u / s.split];
-    const uint32_t part = u % s.split;
-    if (s.split == 1) return d;
-    if (d.c >> 31) {
-      if (part) d = Unit{d.a, d.a, 0u, 0u};  // an empty tile
-      return d;
-    }
-    const uint32_t rows = d.b - d.a;
-    const uint32_t a = d.a + rows * part / s.split, b = d.a + rows * (part + 1) / s.split;
-    const uint32_t lo = __ldg(s.off + a);
-    return Unit{a, b, __ldg(s.off + b) - lo, lo};
-  };
   Unit ahead{};
-  if (warp < parts) ahead = part_of(warp);
-  for (uint32_t u = warp; u < parts; u += warps) {
+  if (warp < s.unit_count) ahead = s.units[warp];
+  for (uint32_t u = warp; u < s.unit_count; u += warps) {
     const Unit unit = ahead;
-    if (u + warps < parts) {
-      ahead = part_of(u + warps);
+    if (u + warps < s.unit_count) {
+      ahead = s.units[u + warps];
       if (32 * lane < unit_count(ahead))  // its targets into L2 meanwhile
         asm volatile("prefetch.global.L2 [%0];" ::"l"(s.tgt + unit_first(ahead) + 32 * lane));
     }
@@ -321,6 +516,19 @@ __global__ void __launch_bounds__(32 * kMp32Warps, 5) mp32_iter_kernel(Mp32 s, u
   if (fell_cols) atomicOr(s.fell + ((C * lane) >> 5), fell_cols << ((C * lane) & 31));
 }
 
+// Whether a pass of 64 columns runs mp32_iter_kernel: where a quarter of the
+// units are pieces of long rows and there is one for every second warp of the
+// chip.  Its warp settles a tile's rows one after another, so tiles of short
+// rows and graphs of a unit a warp lose by it (45 searches over a G(n, m) of
+// 24,947 nodes with rows of 14: 675 µs in tiles, 749 so; 71 over one of 17,533:
+// 1,066 and 1,289), and pieces, which are all gathers, gain (128 searches over
+// R-MAT 20: 15.0 and 11.8 ms; 64 over R-MAT 16 with rows of 8: 744 and 650 µs).
+// Rows of 32 columns stay in tiles, four columns a lane (32 searches over an
+// R-MAT of 120,000 nodes: 633 µs, 950 with one column a lane).
+inline bool mp32_rows(const Schedule& s) {
+  return 4ull * (s.count - s.tiles) >= s.count && s.count >= (uint32_t)max_blocks((int)kMp32Blocks) * kMp32Warps / 2;
+}
+
 // Copies the rows that fell into the iterate; clears the bitmap the
 // iteration read (the next iteration writes it).
 template <int P>
@@ -421,19 +629,23 @@ wc_status mp32_pass(Ctx& ctx, const uint64_t* sources, const uint32_t* caps, con
   cudaStream_t st = ctx.stream;
   note_launch(), mp32_seed_kernel<P><<<max_blocks(4), 256, 0, st>>>(s, sources);
   note_launch(), mp32_sources_kernel<P><<<1, 128, 0, st>>>(s, sources);
-  // A graph of fewer units than the chip holds warps has each tile's rows dealt
-  // to up to four (a warp's sixteen batches of a whole tile are what such an
-  // iteration waits for: 71 searches over 17,533 nodes, 1.29 ms undealt).
-  s.split = std::max<uint32_t>(
-      1, std::min<uint32_t>(4, max_blocks((int)blocks_per_sm) * kMp32Warps /
-                                   std::max<uint32_t>(1, csc.schedule.count)));
-  const uint64_t parts = (uint64_t)csc.schedule.count * s.split;
-  const uint32_t grid = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(
-      max_blocks((int)blocks_per_sm), (parts + kMp32Warps - 1) / kMp32Warps));
+  const uint32_t units = csc.schedule.count;
+  const bool rows = P == 64 && mp32_rows(csc.schedule);
+  const size_t smem = 8 * sizeof(Mp32Smem<P>);
+  static const cudaError_t attr = cudaFuncSetAttribute(
+      mp32_tile_kernel<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (attr != cudaSuccess) return cuda_status(attr, ctx.detail, "min-plus kernel attributes");
+  const uint32_t warps = rows ? kMp32Warps : 8;
+  const uint32_t grid = std::max<uint32_t>(1, std::min<uint32_t>(
+      max_blocks(rows ? (int)blocks_per_sm : P == 64 ? 2 : 3), (units + warps - 1) / warps));
   const uint32_t apply_grid = std::max<uint32_t>(1, std::min<uint32_t>(
       max_blocks(8), (uint32_t)((words + 7) / 8)));
   for (uint32_t it = 0; it < max_cap; it++) {
-    note_launch(), mp32_iter_kernel<P><<<grid, 32 * kMp32Warps, 0, st>>>(s, it);
+    if (rows) {
+      note_launch(), mp32_iter_kernel<64><<<grid, 32 * kMp32Warps, 0, st>>>(s, it);
+    } else {
+      note_launch(), mp32_tile_kernel<P><<<grid, 256, smem, st>>>(s, it);
+    }
     note_launch(), mp32_apply_kernel<P><<<apply_grid, 256, 0, st>>>(s, it);
     note_launch(), mp32_control_kernel<P><<<1, 32, 0, st>>>(s, it);
   }
