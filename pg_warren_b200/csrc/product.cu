@@ -125,6 +125,12 @@ static wc_status product(wc_version* v, const wc_call* call, const wc_product* p
     L.unit_count = uc[part + 1] - uc[part];
     L.lanes = nullptr;  // a range of the rows: over the row-split schedule
   }
+  // Under a million entries in rows of fewer than eight, the row-split schedule
+  // too: the lane-major copy's one block of 24 warps an SM is late to start and
+  // a warp's slice is over in a few steps (f64 plus_times, lanes and schedule:
+  // G(n, m) of 5,000 nodes and 30,000 entries 42 and 36 µs, R-MAT of 160,000
+  // nodes and 960,000 entries 55 and 47; R-MAT 16 with rows of 16 45 and 56).
+  if (v->m < (1u << 20) && v->m < 8 * v->n) L.lanes = nullptr;
   if (width > 1) {
     DevBuf* mc;
     WC_TRY(ctx.scratch(POOL_SPMM_CARRY,
