@@ -522,7 +522,8 @@ __global__ void __launch_bounds__(32 * kMp32Warps, 5) mp32_iter_kernel(Mp32 s, u
 // rows and graphs of a unit a warp lose by it (45 searches over a G(n, m) of
 // 24,947 nodes with rows of 14: 675 µs in tiles, 749 so; 71 over one of 17,533:
 // 1,066 and 1,289), and pieces, which are all gathers, gain (128 searches over
-// R-MAT 20: 15.0 and 11.8 ms; 64 over R-MAT 16 with rows of 8: 744 and 650 µs).
+// R-MAT 20: 15.0 and 11.8 ms).  The line is on the safe side: 64 over R-MAT 16
+// with rows of 8, which lies just under it, take 728 µs in tiles and 650 so.
 // Rows of 32 columns stay in tiles, four columns a lane (32 searches over an
 // R-MAT of 120,000 nodes: 633 µs, 950 with one column a lane).
 inline bool mp32_rows(const Schedule& s) {
