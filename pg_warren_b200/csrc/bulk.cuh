@@ -41,6 +41,14 @@ __device__ inline uint64_t l2_evict_first_policy() {
   return p;
 }
 
+// An L2 policy under which the lines are kept longest: for the vector the
+// gathers of a pull re-read (its values are read once per entry).
+__device__ inline uint64_t l2_evict_last_policy() {
+  uint64_t p;
+  asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(p));
+  return p;
+}
+
 // Global → shared bulk copy of `bytes` (a multiple of 16, both addresses
 // 16-byte aligned), completing its bytes on `bar`.
 __device__ inline void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {

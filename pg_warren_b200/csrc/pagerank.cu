@@ -348,10 +348,20 @@ __global__ void __launch_bounds__(kLaneThreads, 1)
   if (reduce_two(delta, dangling, s.partials, s.counter, more)) pr_close(s, it, delta, dangling);
 }
 
-// One iteration over a range of the row-split schedule of the
-// locality-ordered CSC (a part of a row-partitioned solve).  Unweighted, four
-// blocks an SM (64 registers) keep more gathers in flight; with weights the
-// extra registers would spill, so three.
+// The messages that pr_iter_kernel's gathers keep in L1: 64 KB of them, what
+// the SM's L1 holds beside four blocks' staging rings.  They are those of the
+// rows numbered first, the longest, which a graph of skewed degrees gathers
+// most often as well.
+constexpr uint32_t kHotRows = 8192;
+
+// One iteration over a range of the row-split schedule of the CSC in row
+// order (a part of a row-partitioned solve).  Unweighted, four blocks an SM
+// (64 registers) keep more gathers in flight; with weights the extra
+// registers would spill, so three.  Bound by the latency of the gathers; with
+// plain loads in place of load_x_split's the parts of a weighted R-MAT 22 took
+// 1.05 ms whole and 0.30, 0.32 and 0.37 (first, second and last quarter), with
+// the split 0.97 and 0.29, 0.30 and 0.34 (an unweighted one 0.70 and 0.71
+// whole).
 template <class W>
 __global__ void __launch_bounds__(kPullThreads, WSize<W>::v == 0 ? 4 : 3)
     pr_iter_kernel(CsrView<W> A, PrState s, uint32_t it) {
@@ -361,7 +371,7 @@ __global__ void __launch_bounds__(kPullThreads, WSize<W>::v == 0 ? 4 : 3)
   const int cur = it & 1;
   PrEpi epi(&s, cur, s.dangling[it]);
   PullRing<double, W>* ring = reinterpret_cast<PullRing<double, W>*>(smem) + (threadIdx.x >> 5);
-  pull_units<double, WC_PLUS_TIMES, W>(A, s.msg[cur], epi, s.err, ring);
+  pull_units<double, WC_PLUS_TIMES, W, PrEpi, true>(A, s.msg[cur], epi, s.err, ring);
   pr_pass_cancel(s, cancel);
   double delta = epi.delta, dangling = epi.dangling_out;
   if (reduce_two(delta, dangling, s.partials, s.counter)) pr_close(s, it, delta, dangling);
@@ -385,7 +395,7 @@ static wc_status launch_iter(const PullLaunch& L, const PrState& s, uint32_t it,
 template <class W>
 static wc_status launch_part(const PullLaunch& L, const PrState& s, uint32_t it, uint32_t blocks) {
   CsrView<W> A{L.off, L.tgt, static_cast<const W*>(L.weights), L.units, L.unit_count, L.counters,
-               L.carry};
+               L.carry, kHotRows};
   constexpr size_t smem = pull_smem_bytes<double, W>();
   static const cudaError_t attr = cudaFuncSetAttribute(
       pr_iter_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

@@ -40,6 +40,7 @@ template <class W> struct CsrView {
   uint32_t unit_count;
   uint32_t* counters;
   void* carry;
+  uint32_t hot = 0;  // with SPLIT: the rows whose values L1 keeps
 };
 template <> struct CsrView<void> {
   const uint32_t* off;
@@ -49,6 +50,7 @@ template <> struct CsrView<void> {
   uint32_t unit_count;
   uint32_t* counters;
   void* carry;
+  uint32_t hot = 0;  // with SPLIT: the rows whose values L1 keeps
 };
 
 // An entry's weight as stored (WT), loaded apart from its product so the
@@ -84,6 +86,28 @@ template <class E, int S> struct EntryOf<E, S, void> {
 template <class E> __device__ inline E load_x(const E* x, uint32_t j) { return __ldg(x + j); }
 template <> __device__ inline bool8 load_x<bool8>(const bool8* x, uint32_t j) {
   return *(x + j);
+}
+
+// The gather of a solver's own vector, which every iteration reads again: of
+// the rows numbered below `hot` through L1, of the others past it, so that
+// they do not evict those; in L2 every value is kept ahead of the streamed CSR
+// (`keep`: an l2_evict_last_policy).  8-byte elements only; others take load_x.
+template <class E>
+__device__ inline E load_x_split(const E* x, uint32_t j, uint32_t hot, uint64_t keep) {
+  if constexpr (sizeof(E) == 8) {
+    unsigned long long b;
+    if (j < hot)
+      asm("ld.global.nc.L1::evict_last.L2::cache_hint.b64 %0, [%1], %2;"
+          : "=l"(b) : "l"(x + j), "l"(keep));
+    else
+      asm("ld.global.nc.L1::no_allocate.L2::cache_hint.b64 %0, [%1], %2;"
+          : "=l"(b) : "l"(x + j), "l"(keep));
+    E v;
+    memcpy(&v, &b, 8);
+    return v;
+  } else {
+    return load_x(x, j);
+  }
 }
 
 // An accumulator with a presence flag: the first entry sets the sum.
@@ -226,10 +250,10 @@ __device__ inline typename EntryOf<E, S, W>::WT ring_weight(const PullRing<E, W>
 // Stages the products of the unit in buffer b (count <= 256 entries) in the
 // warp's stage: each lane gathers its (up to 8) x values at once, then forms
 // the products.
-template <class E, int S, class W>
+template <class E, int S, class W, bool SPLIT>
 __device__ inline void stage_products(const PullRing<E, W>* ring, int b, const E* __restrict__ x,
                                       uint32_t e0, uint32_t count, E* stage, DeviceError* err,
-                                      uint32_t row) {
+                                      uint32_t row, uint32_t hot, uint64_t keep) {
   const unsigned lane = threadIdx.x & 31;
   constexpr int Q = kTileEntries / 32;
   const uint32_t* tg = ring->tgt[b] + (e0 & 3u);
@@ -237,7 +261,10 @@ __device__ inline void stage_products(const PullRing<E, W>* ring, int b, const E
 #pragma unroll
   for (int q = 0; q < Q; q++) {
     const uint32_t k = lane + 32 * q;
-    if (k < count) xv[q] = load_x(x, tg[k]);
+    if (k < count) {
+      if constexpr (SPLIT) xv[q] = load_x_split(x, tg[k], hot, keep);
+      else xv[q] = load_x(x, tg[k]);
+    }
   }
 #pragma unroll
   for (int q = 0; q < Q; q++) {
@@ -252,12 +279,13 @@ __device__ inline void stage_products(const PullRing<E, W>* ring, int b, const E
 }
 
 // Walks the schedule, a warp per unit, the units of a warp strided by the
-// grid's warp count, through the warp's staging ring.  The epilogue's
+// grid's warp count, through the warp's staging ring.  SPLIT: A.hot splits
+// the gathers (load_x_split).  The epilogue's
 // per-row operands (`epi.pre(row)`) are requested as a unit starts, so they
 // arrive with its gathers.  `epi.row(row, present, value, pre)` is called
 // exactly once per row, by one lane.  A ring wait that runs out (about 2 s)
 // raises WC_DEVICE_TIMEOUT and ends the walk after the copies in flight.
-template <class E, int S, class W, class Epi>
+template <class E, int S, class W, class Epi, bool SPLIT = false>
 __device__ inline void pull_units(const CsrView<W>& A, const E* __restrict__ x, Epi& epi,
                                   DeviceError* err, PullRing<E, W>* ring) {
   constexpr int R = PullRing<E, W>::R;
@@ -272,6 +300,8 @@ __device__ inline void pull_units(const CsrView<W>& A, const E* __restrict__ x, 
     for (int b = 0; b < R; b++) mbar_init(&ring->bar[b], 1);
   __syncwarp();
   const uint64_t stream = l2_evict_first_policy();
+  uint64_t keep = 0;
+  if constexpr (SPLIT) keep = l2_evict_last_policy();
   Unit ahead{0u, 0u, 0u, 0u};  // lane 0: the next unit to issue
   uint32_t pending = 0;        // buffers with a copy in flight (uniform)
   for (int b = 0; b < R; b++) {
@@ -309,7 +339,7 @@ __device__ inline void pull_units(const CsrView<W>& A, const E* __restrict__ x, 
         hi = soff[lane + 1];
         pre = epi.pre(r0 + lane);
       }
-      stage_products<E, S, W>(ring, b, x, e0, count, ring->stage, err, r0);
+      stage_products<E, S, W, SPLIT>(ring, b, x, e0, count, ring->stage, err, r0, A.hot, keep);
       __syncwarp();
       if (lane < rows) {
         E sum{};
@@ -334,7 +364,7 @@ __device__ inline void pull_units(const CsrView<W>& A, const E* __restrict__ x, 
       const uint32_t row = unit.a, e0 = unit.b, e1 = unit.d;
       const uint32_t slot = unit.c & 0x7fffffffu;
       const uint32_t count = e1 - e0;
-      stage_products<E, S, W>(ring, b, x, e0, count, ring->stage, err, row);
+      stage_products<E, S, W, SPLIT>(ring, b, x, e0, count, ring->stage, err, row, A.hot, keep);
       __syncwarp();
       Partial<E, ADD> mine{Acc<E, ADD>::of(E{}), false};
       constexpr uint32_t per = kTileEntries / 32;
