@@ -226,6 +226,7 @@ struct PrEpi {
   // dangling · start and teleport · start, and whether neither failed.
   double uniform_dp = 0.0, uniform_b = 0.0;
   bool uniform_ok = false;
+  bool slots = true;  // whether a row's slot takes what it adds to the sums
   __device__ PrEpi(const PrState* st, int c, double in) : s(st), cur(c), dangling_in(in) {
     uniform_ok = sql_float<F_MUL>(in, st->start, &uniform_dp) == 0 &&
                  sql_float<F_MUL>(st->teleport, st->start, &uniform_b) == 0;
@@ -262,7 +263,7 @@ struct PrEpi {
     const double change = fabs(next - pr.old);
     st.x[cur ^ 1][i] = next;
     const double dangles = spread_row(next, pr.out, &st.msg[cur ^ 1][i], st.err, i);
-    if (slot) {
+    if (slots && slot) {
       static_assert(sizeof(Slot) == sizeof(double2), "a slot holds the row's two sums");
       *reinterpret_cast<double2*>(slot) = make_double2(change, dangles);
     } else {
@@ -318,6 +319,33 @@ template <class W> static LaneView<W> ranked_view(const PullLaunch& L, const wc_
   return A;
 }
 
+// The rows that several warps' pieces make up, [lo, hi) of `longs` (row, first
+// slot, pieces) with more than `run` pieces, left their shares of the sums in
+// their slots: each thread of the last block adds some, in row order, four
+// loads in flight.
+__device__ inline void add_slots(double& a, double& b, const uint4* longs, uint32_t lo,
+                                 uint32_t hi, uint32_t run, const PrEpi::Slot* carry) {
+  constexpr uint32_t U = 4;
+  for (uint64_t r0 = lo + threadIdx.x; r0 < hi; r0 += U * blockDim.x) {
+    uint4 L[U];
+    double2 v[U];
+#pragma unroll
+    for (uint32_t q = 0; q < U; q++) {
+      const uint64_t r = r0 + q * blockDim.x;
+      L[q] = r < hi ? __ldg(longs + r) : make_uint4(0u, 0u, 0u, 0u);
+    }
+#pragma unroll
+    for (uint32_t q = 0; q < U; q++)
+      if (L[q].z > run) v[q] = __ldcg(reinterpret_cast<const double2*>(carry + L[q].y));
+#pragma unroll
+    for (uint32_t q = 0; q < U; q++)
+      if (L[q].z > run) {
+        a += v[q].x;
+        b += v[q].y;
+      }
+  }
+}
+
 // One iteration over the reverse CSR's lane-major copy: one launch, one
 // block an SM.
 template <class W>
@@ -334,16 +362,8 @@ __global__ void __launch_bounds__(kLaneThreads, 1)
   lane_units<double, WC_PLUS_TIMES, W>(A, s.msg[cur], pr_hot, epi, s.err);
   pr_pass_cancel(s, cancel);
   double delta = epi.delta, dangling = epi.dangling_out;
-  // The rows of several units left their shares of the sums in their slots.
   auto more = [&](double& a, double& b) {
-    for (uint32_t r = threadIdx.x; r < long_count; r += blockDim.x) {
-      const uint4 L = __ldg(longs + r);  // row, first slot, pieces
-      if (L.z <= run) continue;
-      const double2 v = __ldcg(reinterpret_cast<const double2*>(
-          static_cast<const PrEpi::Slot*>(A.carry) + L.y));
-      a += v.x;
-      b += v.y;
-    }
+    add_slots(a, b, longs, 0, long_count, run, static_cast<const PrEpi::Slot*>(A.carry));
   };
   if (reduce_two(delta, dangling, s.partials, s.counter, more)) pr_close(s, it, delta, dangling);
 }
@@ -354,8 +374,9 @@ __global__ void __launch_bounds__(kLaneThreads, 1)
 // most often as well.
 constexpr uint32_t kHotRows = 8192;
 
-// One iteration over a range of the row-split schedule of the CSC in row
-// order (a part of a row-partitioned solve).  Unweighted, four blocks an SM
+// One iteration over the row-split schedule of the CSC in row order (lanes_pay
+// says when), or over a range of it (a part of a row-partitioned solve, which
+// gives no `longs`: its sums take a row in pieces as it comes).  Unweighted, four blocks an SM
 // (64 registers) keep more gathers in flight; with weights the extra
 // registers would spill, so three.  Bound by the latency of the gathers; with
 // plain loads in place of load_x_split's the parts of a weighted R-MAT 22 took
@@ -364,17 +385,21 @@ constexpr uint32_t kHotRows = 8192;
 // whole).
 template <class W>
 __global__ void __launch_bounds__(kPullThreads, WSize<W>::v == 0 ? 4 : 3)
-    pr_iter_kernel(CsrView<W> A, PrState s, uint32_t it) {
+    pr_iter_kernel(CsrView<W> A, PrState s, uint32_t it, const uint4* longs, uint32_t long_count) {
   extern __shared__ __align__(16) unsigned char smem[];
   if (*(volatile int32_t*)s.done) return;
   const int32_t cancel = pr_read_cancel(s);
   const int cur = it & 1;
   PrEpi epi(&s, cur, s.dangling[it]);
+  epi.slots = longs != nullptr;
   PullRing<double, W>* ring = reinterpret_cast<PullRing<double, W>*>(smem) + (threadIdx.x >> 5);
   pull_units<double, WC_PLUS_TIMES, W, PrEpi, true>(A, s.msg[cur], epi, s.err, ring);
   pr_pass_cancel(s, cancel);
   double delta = epi.delta, dangling = epi.dangling_out;
-  if (reduce_two(delta, dangling, s.partials, s.counter)) pr_close(s, it, delta, dangling);
+  auto more = [&](double& a, double& b) {
+    add_slots(a, b, longs, 0, long_count, 0, static_cast<const PrEpi::Slot*>(A.carry));
+  };
+  if (reduce_two(delta, dangling, s.partials, s.counter, more)) pr_close(s, it, delta, dangling);
 }
 
 template <class W>
@@ -393,14 +418,16 @@ static wc_status launch_iter(const PullLaunch& L, const PrState& s, uint32_t it,
 }
 
 template <class W>
-static wc_status launch_part(const PullLaunch& L, const PrState& s, uint32_t it, uint32_t blocks) {
+static wc_status launch_rows(const PullLaunch& L, const PrState& s, uint32_t it, uint32_t blocks,
+                             const Schedule* longs) {
   CsrView<W> A{L.off, L.tgt, static_cast<const W*>(L.weights), L.units, L.unit_count, L.counters,
                L.carry, kHotRows};
   constexpr size_t smem = pull_smem_bytes<double, W>();
   static const cudaError_t attr = cudaFuncSetAttribute(
       pr_iter_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (attr != cudaSuccess) return cuda_status(attr, L.detail, "pagerank kernel attributes");
-  note_launch(), pr_iter_kernel<W><<<blocks, kPullThreads, smem, L.stream>>>(A, s, it);
+  note_launch(), pr_iter_kernel<W><<<blocks, kPullThreads, smem, L.stream>>>(
+      A, s, it, longs ? longs->long_list.as<uint4>() : nullptr, longs ? longs->long_rows : 0);
   return WC_OK;
 }
 
@@ -413,10 +440,10 @@ wc_status launch_pr_init(const PrState& s, uint32_t grid, cudaStream_t stream) {
   return cuda_status(cudaGetLastError(), nullptr, "pagerank init");
 }
 
-wc_status launch_part_iteration(const PullLaunch& L, const PrState& s, uint32_t it,
-                                uint32_t blocks) {
-  if (L.weight_kind == WEIGHTS_F64) return launch_part<double>(L, s, it, blocks);
-  return launch_part<void>(L, s, it, blocks);
+wc_status launch_row_iteration(const PullLaunch& L, const PrState& s, uint32_t it, uint32_t blocks,
+                               const Schedule* longs) {
+  if (L.weight_kind == WEIGHTS_F64) return launch_rows<double>(L, s, it, blocks, longs);
+  return launch_rows<void>(L, s, it, blocks, longs);
 }
 
 uint64_t live_count(const uint64_t* tomb, uint64_t n) {
@@ -558,13 +585,32 @@ wc_status PageRankRun::out_now(Ctx& ctx) {
   return cuda_status(cudaGetLastError(), ctx.detail, "out-degrees");
 }
 
+// Whether a solve walks the lane-major copy.  Over a skewed graph (one with
+// long rows) of few entries its longest slices are what an iteration waits
+// for, and the row-split schedule, whose units are all alike, is the faster.
+// Solves to 1e-10 over R-MAT graphs of so many nodes and edges, lanes and
+// schedule, µs: 4,096 and 28,700 386 and 271 (weighted 440 and 302), 33,000 and
+// 157,396 490 and 326 (511 and 340), 65,536 and 954,361 339 and 334 (366 and
+// 383), 131,072 and 999,085 468 and 411 (519 and 486), 262,144 and 1,024,319
+// 558 and 506.  In longer rows the schedule holds out further: 65,536 and
+// 1,818,513 512 and 397, 131,072 and 1,942,324 541 and 474 (weighted 611 and
+// 615), but 262,144 and 2,016,841 554 and 568, 524,288 and 2,057,684 620 and
+// 663.  G(n, m) graphs have no long row: 65,536 and 262,129 260 and 290.
+static bool lanes_pay(const wc_version* v, bool weighted) {
+  if (!v->rev.schedule.long_rows) return true;
+  return v->m >= (!weighted && v->m >= 12 * v->n ? 1u << 21 : 1u << 20);
+}
+
 wc_status PageRankRun::run(Ctx& ctx) {
   wc_version* v = ctx.v;
   WC_TRY(launch_pr_init(s, grid, ctx.stream));
   PullLaunch L;
   WC_TRY(prepare_pull(ctx, v->rev, WC_PLUS_TIMES, opts.weighted, WC_F64, 1, L));
+  const bool lanes = L.lanes && lanes_pay(v, L.weight_kind == WEIGHTS_F64);
+  if (!lanes)
+    WC_TRY(prepare_pull(ctx, v->loc.csc, WC_PLUS_TIMES, opts.weighted, WC_F64, 1, L));
   // No more blocks than the step keeps sums for.
-  const uint32_t blocks = L.lanes ? std::min(lane_grid(L), grid) : 0;
+  const uint32_t blocks = lanes ? std::min(lane_grid(L), grid) : grid;
   // With a tolerance the solve usually stops well before max_iter: the
   // host keeps at most kAhead iterations queued beyond the last one the
   // device reported, and stops queueing once the device reports the stop,
@@ -576,7 +622,7 @@ wc_status PageRankRun::run(Ctx& ctx) {
     pace[1] = 0;
   }
   ctx.phase_begin("iteration");
-  for (uint32_t it = 0; L.lanes && it < opts.max_iter; it++) {
+  for (uint32_t it = 0; it < opts.max_iter; it++) {
     // A cancel stops the queueing (the kernels queued read the device's
     // copy of the word, which finish() raises).
     if (ctx.cancelled()) break;
@@ -588,7 +634,8 @@ wc_status PageRankRun::run(Ctx& ctx) {
       }
       if (stop) break;
     }
-    if (L.weight_kind == WEIGHTS_F64) WC_TRY(launch_iter<double>(L, s, it, blocks, v));
+    if (!lanes) WC_TRY(launch_row_iteration(L, s, it, blocks, &v->loc.csc.schedule));
+    else if (L.weight_kind == WEIGHTS_F64) WC_TRY(launch_iter<double>(L, s, it, blocks, v));
     else WC_TRY(launch_iter<void>(L, s, it, blocks, v));
   }
   ctx.phase_end();

@@ -54,10 +54,11 @@ struct PageRankRun {
 uint64_t live_count(const uint64_t* tomb, uint64_t n);
 // pr_init_kernel: the start vector, its messages and dangling rank.
 wc_status launch_pr_init(const PrState& s, uint32_t grid, cudaStream_t stream);
-// One iteration (pr_iter_kernel) over L's units.
+// One iteration (pr_iter_kernel) over L's units; `longs`, for all of them: the
+// schedule's long rows, whose shares of the sums are then added in row order.
 struct PullLaunch;
-wc_status launch_part_iteration(const PullLaunch& L, const PrState& s, uint32_t it,
-                                uint32_t blocks);
+wc_status launch_row_iteration(const PullLaunch& L, const PrState& s, uint32_t it, uint32_t blocks,
+                               const Schedule* longs);
 // Drops a version's partitioned solve (wc_pagerank_part_*) when it is released.
 void pagerank_part_forget(const wc_version* v);
 // The row-partitioned search's and product's state kept with a version

@@ -205,7 +205,7 @@ wc_status wc_pagerank_part_step(wc_version* v, const wc_call* call, uint32_t ite
   WC_TRY(prepare_pull(ctx, v->loc.csc, WC_PLUS_TIMES, run.opts.weighted, WC_F64, 1, L));
   L.units += ps->unit_begin;
   L.unit_count = ps->unit_end - ps->unit_begin;
-  if (L.unit_count) WC_TRY(launch_part_iteration(L, run.s, iteration, run.grid));
+  if (L.unit_count) WC_TRY(launch_row_iteration(L, run.s, iteration, run.grid, nullptr));
   WC_TRY(ctx.finish());
   double host[2] = {0.0, 0.0};
   if (L.unit_count) {

@@ -283,7 +283,8 @@ __device__ inline void stage_products(const PullRing<E, W>* ring, int b, const E
 // the gathers (load_x_split).  The epilogue's
 // per-row operands (`epi.pre(row)`) are requested as a unit starts, so they
 // arrive with its gathers.  `epi.row(row, present, value, pre)` is called
-// exactly once per row, by one lane.  A ring wait that runs out (about 2 s)
+// exactly once per row, by one lane; of a row in pieces, which whichever warp
+// came last finishes, with the row's first carry slot, read by then.  A ring wait that runs out (about 2 s)
 // raises WC_DEVICE_TIMEOUT and ends the walk after the copies in flight.
 template <class E, int S, class W, class Epi, bool SPLIT = false>
 __device__ inline void pull_units(const CsrView<W>& A, const E* __restrict__ x, Epi& epi,
@@ -394,7 +395,7 @@ __device__ inline void pull_units(const CsrView<W>& A, const E* __restrict__ x, 
           E v;
           int32_t s = total.acc.value(&v);
           if (s) raise(err, s, row);
-          epi.row(row, true, v, pre);
+          epi.row(row, true, v, pre, carry + first);
         }
       }
     }
