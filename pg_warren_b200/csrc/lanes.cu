@@ -156,7 +156,7 @@ __global__ void lane_entries_kernel(const LaneUnit* units, uint32_t count, const
 }
 
 wc_status device_lanes(wc_version* v, DevCsr& d, const std::vector<uint64_t>& off,
-                       const DevCsr& other, wc_error_detail* detail) {
+                       const DevCsr& other, uint64_t& room, wc_error_detail* detail) {
   const uint64_t n = v->n, m = v->m;
   cudaStream_t st = v->stream;
   LaneCsr& L = d.lanes;
@@ -211,6 +211,10 @@ wc_status device_lanes(wc_version* v, DevCsr& d, const std::vector<uint64_t>& of
   const uint64_t places = L.places =
       (uint64_t)first * 32 + (m - long_entries) + 32 * cap + 1024 + 32 * (uint64_t)cls.slice[1];
   L.hot_count = n < kHotTarget ? (uint32_t)std::min<uint64_t>(hot_nodes, kHotSlots) : 0;
+  const uint64_t bytes = L.count * sizeof(LaneUnit) + n * 4 + shorts * 2ull +
+                         places * (4 + (d.weights.ptr ? 8 : 0) + (d.iweights.ptr ? 4 : 0));
+  if (bytes > room) return WC_OUT_OF_MEMORY;
+  room -= bytes;
   WC_TRY(L.units.alloc(v->budget, std::max<uint64_t>(L.count, 1) * sizeof(LaneUnit), detail));
   WC_TRY(L.rows.alloc(v->budget, std::max<uint64_t>(n, 1) * 4, detail));
   WC_TRY(L.lengths.alloc(v->budget, std::max<uint32_t>(shorts, 1) * 2, detail));

@@ -91,9 +91,6 @@ wc_status device_locality(wc_version* v, wc_error_detail* detail) {
   WC_TRY(c.targets.alloc(v->budget, m * 4 + kBulkPad, detail));
   if (v->weighted) WC_TRY(c.weights.alloc(v->budget, m * 8 + kBulkPad, detail));
   if (v->weighted && v->integral) WC_TRY(c.iweights.alloc(v->budget, m * 4 + kBulkPad, detail));
-  const LaneCsr& lanes = v->rev.lanes;
-  WC_TRY(L.lane_targets.alloc(v->budget, lanes.places * 4, detail));
-  if (lanes.hot_count) WC_TRY(L.lane_hot.alloc(v->budget, lanes.hot_count * 4, detail));
   if (n) {
     // Order: a stable radix sort of (¬length, id).
     DevBuf k0, k1, i1, temp;
@@ -134,9 +131,6 @@ wc_status device_locality(wc_version* v, wc_error_detail* detail) {
           v->rev.targets.as<uint32_t>(), v->weighted ? v->rev.weights.as<double>() : nullptr,
           c.iweights.ptr ? v->rev.iweights.as<int32_t>() : nullptr, c.offsets.as<uint32_t>(),
           (uint32_t)n, c.targets.as<uint32_t>(), c.weights.as<double>(), c.iweights.as<int32_t>());
-    note_launch(), loc_lanes_kernel<<<grid_of(lanes.places), 256, 0, st>>>(
-        lanes.targets.as<uint32_t>(), lanes.places, lanes.hot.as<uint32_t>(), lanes.hot_count,
-        L.perm.as<uint32_t>(), L.lane_targets.as<uint32_t>(), L.lane_hot.as<uint32_t>());
     WC_CUDA(cudaStreamSynchronize(st), detail);  // before the transient buffers go
   } else {
     WC_CUDA(cudaMemsetAsync(c.offsets.ptr, 0, 4, st), detail);
@@ -148,6 +142,22 @@ wc_status device_locality(wc_version* v, wc_error_detail* detail) {
   std::vector<uint64_t> off(off32.begin(), off32.end());
   WC_TRY(put_schedule(v, c, off, detail));
   return cuda_status(cudaGetLastError(), detail, "locality order");
+}
+
+wc_status device_lane_numbers(wc_version* v, uint64_t& room, wc_error_detail* detail) {
+  const LaneCsr& lanes = v->rev.lanes;
+  Locality& L = v->loc;
+  if (!lanes.places) return WC_OK;  // no copy, or no nodes
+  const uint64_t bytes = (lanes.places + lanes.hot_count) * 4;
+  if (bytes > room) return WC_OUT_OF_MEMORY;
+  WC_TRY(L.lane_targets.alloc(v->budget, lanes.places * 4, detail));
+  if (lanes.hot_count) WC_TRY(L.lane_hot.alloc(v->budget, lanes.hot_count * 4, detail));
+  room -= bytes;
+  if (v->n)
+    note_launch(), loc_lanes_kernel<<<grid_of(lanes.places), 256, 0, v->stream>>>(
+        lanes.targets.as<uint32_t>(), lanes.places, lanes.hot.as<uint32_t>(), lanes.hot_count,
+        L.perm.as<uint32_t>(), L.lane_targets.as<uint32_t>(), L.lane_hot.as<uint32_t>());
+  return cuda_status(cudaStreamSynchronize(v->stream), detail, "lane-major numbers");
 }
 
 // ------------------------------------------------- renumbering vectors

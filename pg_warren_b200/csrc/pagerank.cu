@@ -606,7 +606,8 @@ wc_status PageRankRun::run(Ctx& ctx) {
   WC_TRY(launch_pr_init(s, grid, ctx.stream));
   PullLaunch L;
   WC_TRY(prepare_pull(ctx, v->rev, WC_PLUS_TIMES, opts.weighted, WC_F64, 1, L));
-  const bool lanes = L.lanes && lanes_pay(v, L.weight_kind == WEIGHTS_F64);
+  const bool lanes =
+      L.lanes && v->loc.lane_targets.ptr && lanes_pay(v, L.weight_kind == WEIGHTS_F64);
   if (!lanes)
     WC_TRY(prepare_pull(ctx, v->loc.csc, WC_PLUS_TIMES, opts.weighted, WC_F64, 1, L));
   // No more blocks than the step keeps sums for.

@@ -236,12 +236,14 @@ struct Schedule {
   DevBuf counters;    // u32[slots]: arrivals per long row (indexed by its first slot)
   DevBuf carry;       // the pieces' partial results, kCarryBytesPerSlot per slot
   DevBuf long_list;   // uint4[long_rows]: each long row, its first slot and piece count
-  // The reverse CSR's units again, for the batched BFS (count of them): the
-  // long rows' first pieces, the tiles, then the other pieces by their place
-  // in their row, so that a row's later pieces come after its earlier ones
-  // have left their bits.  round_masks: per unit, a tile's rows that hold
-  // entries (bit r: row a + r).
+  // The reverse CSR's units again, for the batched BFS (count of them; none
+  // where there was no room for them): the long rows' first pieces, the tiles,
+  // then the other pieces by their place in their row, so that a row's later
+  // pieces come after its earlier ones have left their bits.  round_masks: per
+  // unit as that search takes them, a tile's rows that hold entries (bit r:
+  // row a + r).
   DevBuf rounds, round_masks;
+  const Unit* batch_units() const { return (rounds.ptr ? rounds : units).as<Unit>(); }
   uint32_t count = 0;
   uint32_t slots = 0;
   uint32_t long_rows = 0;
@@ -285,7 +287,7 @@ struct LaneCsr {
 struct DevCsr {
   DevBuf offsets, targets, weights, iweights;
   Schedule schedule;
-  LaneCsr lanes;  // the version's two orientations only
+  LaneCsr lanes;  // the version's two orientations only, where there is room
   uint32_t max_degree = 0;
 };
 
@@ -294,7 +296,7 @@ struct DevCsr {
 // number and order a new number back to the dense id.
 struct Locality {
   DevBuf perm, order;  // u32[n] each
-  DevBuf lane_targets, lane_hot;  // rev.lanes' targets and hot nodes, renumbered
+  DevBuf lane_targets, lane_hot;  // rev.lanes' targets and hot nodes, renumbered (or none)
   DevCsr csc;
 };
 

@@ -100,7 +100,7 @@ wc_status device_row_masks(wc_version* v, DevCsr& d, wc_error_detail* detail) {
   const uint32_t count = d.schedule.count;
   if (count)
     note_launch(), row_masks_kernel<<<max_blocks(8), 256, 0, v->stream>>>(
-        d.schedule.rounds.as<Unit>(), count, d.offsets.as<uint32_t>(),
+        d.schedule.batch_units(), count, d.offsets.as<uint32_t>(),
         d.schedule.round_masks.as<uint32_t>());
   return cuda_status(cudaStreamSynchronize(v->stream), detail, "row masks");
 }

@@ -110,13 +110,12 @@ static wc_status put_rounds(wc_version* v, DevCsr& d, const std::vector<Unit>& u
   if (!units.empty())
     WC_CUDA(cudaMemcpy(s.rounds.ptr, ordered.data(), ordered.size() * sizeof(Unit),
                        cudaMemcpyHostToDevice), detail);
-  WC_TRY(s.round_masks.alloc(v->budget, std::max<size_t>(units.size(), 1) * 4, detail));
-  return device_row_masks(v, d, detail);
+  return WC_OK;
 }
 
 // The schedule of one orientation from its host offsets.
 wc_status put_schedule(wc_version* v, DevCsr& d, const std::vector<uint64_t>& off,
-                              wc_error_detail* detail) {
+                       wc_error_detail* detail, std::vector<Unit>* units_out) {
   std::vector<Unit> units;
   Schedule& s = d.schedule;
   build_units(v->n, off.data(), units, s.slots, s.long_rows, s.tiles, d.max_degree);
@@ -144,7 +143,54 @@ wc_status put_schedule(wc_version* v, DevCsr& d, const std::vector<uint64_t>& of
   if (!longs.empty())
     WC_CUDA(cudaMemcpy(s.long_list.ptr, longs.data(), longs.size() * 4, cudaMemcpyHostToDevice),
             detail);
-  return &d == &v->rev ? put_rounds(v, d, units, off, detail) : WC_OK;
+  if (&d == &v->rev)
+    WC_TRY(s.round_masks.alloc(v->budget, std::max<size_t>(units.size(), 1) * 4, detail));
+  if (units_out) *units_out = std::move(units);
+  return WC_OK;
+}
+
+// Builds what only makes calls faster: with no room for it a version does
+// without, and its calls take the way that needs none.
+template <class Build>
+static wc_status where_room(wc_error_detail* detail, Build&& build, bool* built) {
+  const wc_error_detail before = detail ? *detail : wc_error_detail{};
+  const wc_status st = build();
+  *built = st == WC_OK;
+  if (st != WC_MEMORY_LIMIT && st != WC_OUT_OF_MEMORY) return st;
+  if (detail) *detail = before;
+  return WC_OK;
+}
+
+// The batched BFS's units and the lane-major copies, the reverse one with its
+// renumbering (PageRank's) first.  They come after everything that a version
+// cannot do without, so that a budget or a device that holds that accepts it,
+// and take at most half of what the device has left, which the rest of the
+// program allocates from too.
+static wc_status put_fast_copies(wc_version* v, const std::vector<Unit>& rev_units,
+                                 wc_error_detail* detail) {
+  bool built = false;
+  WC_TRY(where_room(detail, [&] {
+    return put_rounds(v, v->rev, rev_units, v->host_rev_offsets, detail);
+  }, &built));
+  if (!built) v->rev.schedule.rounds.release();
+  WC_TRY(device_row_masks(v, v->rev, detail));
+  size_t left = 0, total = 0;
+  WC_CUDA(cudaMemGetInfo(&left, &total), detail);
+  uint64_t room = left / 2;
+  WC_TRY(where_room(detail, [&] {
+    return device_lanes(v, v->rev, v->host_rev_offsets, v->fwd, room, detail);
+  }, &built));
+  if (!built) v->rev.lanes = LaneCsr{};
+  WC_TRY(where_room(detail, [&] { return device_lane_numbers(v, room, detail); }, &built));
+  if (!built) {
+    v->loc.lane_targets.release();
+    v->loc.lane_hot.release();
+  }
+  WC_TRY(where_room(detail, [&] {
+    return device_lanes(v, v->fwd, v->host_offsets, v->rev, room, detail);
+  }, &built));
+  if (!built) v->fwd.lanes = LaneCsr{};
+  return WC_OK;
 }
 
 wc_status wc_device_check(wc_error_detail* detail) {
@@ -169,9 +215,8 @@ wc_status finish_version(wc_version* v, wc_error_detail* detail) {
   WC_TRY(device_weight_facts(v, detail));
   WC_TRY(device_symmetric(v, detail));
   WC_TRY(put_schedule(v, v->fwd, v->host_offsets, detail));
-  WC_TRY(put_schedule(v, v->rev, v->host_rev_offsets, detail));
-  WC_TRY(device_lanes(v, v->fwd, v->host_offsets, v->rev, detail));
-  WC_TRY(device_lanes(v, v->rev, v->host_rev_offsets, v->fwd, detail));
+  std::vector<Unit> rev_units;
+  WC_TRY(put_schedule(v, v->rev, v->host_rev_offsets, detail, &rev_units));
   WC_TRY(device_locality(v, detail));
   WC_TRY(v->error.alloc(v->budget, sizeof(DeviceError), detail));
   WC_CUDA(cudaMemset(v->error.ptr, 0, sizeof(DeviceError)), detail);
@@ -184,7 +229,7 @@ wc_status finish_version(wc_version* v, wc_error_detail* detail) {
   v->pace_dev = reinterpret_cast<uint32_t*>(v->cancel_dev + 1);
   WC_CUDA(cudaHostAlloc((void**)&v->stage_host, kStageBytes, cudaHostAllocMapped), detail);
   WC_CUDA(cudaHostGetDevicePointer((void**)&v->stage_dev, v->stage_host, 0), detail);
-  return WC_OK;
+  return put_fast_copies(v, rev_units, detail);
 }
 
 }  // namespace wc
