@@ -159,6 +159,7 @@ wc_status device_lanes(wc_version* v, DevCsr& d, const std::vector<uint64_t>& of
                        const DevCsr& other, uint64_t& room, wc_error_detail* detail) {
   const uint64_t n = v->n, m = v->m;
   cudaStream_t st = v->stream;
+  const Room ask{false};  // no other version's copies for these
   LaneCsr& L = d.lanes;
   const uint32_t shorts = (uint32_t)n - d.schedule.long_rows;
   // Rows by width, the hot nodes, and the long rows' units: runs of pieces,
@@ -174,7 +175,7 @@ wc_status device_lanes(wc_version* v, DevCsr& d, const std::vector<uint64_t>& of
   std::vector<uint4> longs(d.schedule.long_rows);  // row, first slot, pieces
   uint32_t counts[3] = {0, 0, 0};
   DevBuf tally;
-  WC_TRY(tally.alloc(v->budget, sizeof counts, detail));
+  WC_TRY(tally.alloc(v->budget, sizeof counts, detail, ask));
   WC_CUDA(cudaMemsetAsync(tally.ptr, 0, sizeof counts, st), detail);
   if (n)
     note_launch(), lane_counts_kernel<<<grid_of(n), 256, 0, st>>>(
@@ -215,13 +216,13 @@ wc_status device_lanes(wc_version* v, DevCsr& d, const std::vector<uint64_t>& of
                          places * (4 + (d.weights.ptr ? 8 : 0) + (d.iweights.ptr ? 4 : 0));
   if (bytes > room) return WC_OUT_OF_MEMORY;
   room -= bytes;
-  WC_TRY(L.units.alloc(v->budget, std::max<uint64_t>(L.count, 1) * sizeof(LaneUnit), detail));
-  WC_TRY(L.rows.alloc(v->budget, std::max<uint64_t>(n, 1) * 4, detail));
-  WC_TRY(L.lengths.alloc(v->budget, std::max<uint32_t>(shorts, 1) * 2, detail));
-  WC_TRY(L.targets.alloc(v->budget, places * 4, detail));
-  if (d.weights.ptr) WC_TRY(L.weights.alloc(v->budget, places * 8, detail));
-  if (d.iweights.ptr) WC_TRY(L.iweights.alloc(v->budget, places * 4, detail));
-  if (L.hot_count) WC_TRY(L.hot.alloc(v->budget, L.hot_count * 4, detail));
+  WC_TRY(L.units.alloc(v->budget, std::max<uint64_t>(L.count, 1) * sizeof(LaneUnit), detail, ask));
+  WC_TRY(L.rows.alloc(v->budget, std::max<uint64_t>(n, 1) * 4, detail, ask));
+  WC_TRY(L.lengths.alloc(v->budget, std::max<uint32_t>(shorts, 1) * 2, detail, ask));
+  WC_TRY(L.targets.alloc(v->budget, places * 4, detail, ask));
+  if (d.weights.ptr) WC_TRY(L.weights.alloc(v->budget, places * 8, detail, ask));
+  if (d.iweights.ptr) WC_TRY(L.iweights.alloc(v->budget, places * 4, detail, ask));
+  if (L.hot_count) WC_TRY(L.hot.alloc(v->budget, L.hot_count * 4, detail, ask));
   if (!n) return WC_OK;
   // One transient buffer: two key and two id buffers of n words, the sorts'
   // and the scan's temporary memory behind them.  (The rows are sorted into
@@ -239,7 +240,7 @@ wc_status device_lanes(wc_version* v, DevCsr& d, const std::vector<uint64_t>& of
   const uint64_t temp_at = (ids_at + std::max<uint64_t>(words, 2 * slices) + 63) / 64 * 64;
   size_t temp_bytes = std::max<size_t>({sort_bytes, scan_bytes, 16});
   DevBuf transient;
-  WC_TRY(transient.alloc(v->budget, temp_at * 4 + temp_bytes, detail));
+  WC_TRY(transient.alloc(v->budget, temp_at * 4 + temp_bytes, detail, ask));
   uint32_t* k0 = transient.as<uint32_t>();
   uint32_t* ids = k0 + ids_at;
   void* temp = k0 + temp_at;

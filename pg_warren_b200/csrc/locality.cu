@@ -150,8 +150,9 @@ wc_status device_lane_numbers(wc_version* v, uint64_t& room, wc_error_detail* de
   if (!lanes.places) return WC_OK;  // no copy, or no nodes
   const uint64_t bytes = (lanes.places + lanes.hot_count) * 4;
   if (bytes > room) return WC_OUT_OF_MEMORY;
-  WC_TRY(L.lane_targets.alloc(v->budget, lanes.places * 4, detail));
-  if (lanes.hot_count) WC_TRY(L.lane_hot.alloc(v->budget, lanes.hot_count * 4, detail));
+  WC_TRY(L.lane_targets.alloc(v->budget, lanes.places * 4, detail, Room{false}));
+  if (lanes.hot_count)
+    WC_TRY(L.lane_hot.alloc(v->budget, lanes.hot_count * 4, detail, Room{false}));
   room -= bytes;
   if (v->n)
     note_launch(), loc_lanes_kernel<<<grid_of(lanes.places), 256, 0, v->stream>>>(

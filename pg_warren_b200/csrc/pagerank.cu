@@ -682,6 +682,9 @@ wc_status wc_pagerank(wc_version* v, const wc_call* call, const wc_pagerank_opts
   Ctx ctx(v, call);
   if (ctx.cancelled()) return WC_CANCELLED;
   WC_TRY(ctx.begin());
+  // The two ways to walk the rows add the solve's sums in orders of their own:
+  // a solve does not change the way of the next by what it allocates.
+  ctx.keep_lanes = true;
   PageRankRun run;
   ctx.phase_begin("setup");
   WC_TRY(run.setup(ctx, o, tombstones, o->seed));

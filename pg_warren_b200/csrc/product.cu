@@ -54,6 +54,10 @@ wc_status prepare_pull(Ctx& ctx, DevCsr& csr, int semiring, int weighted_flag, i
     }
   }
   L.lanes = csr.lanes.count || csr.lanes.shorts ? &csr.lanes : nullptr;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (L.lanes && ctx.stream && cudaStreamIsCapturing(ctx.stream, &cs) == cudaSuccess &&
+      cs != cudaStreamCaptureStatusNone)
+    v->lanes_captured = true;
   L.units = csr.schedule.units.as<Unit>();
   L.unit_count = csr.schedule.count;
   L.counters = csr.schedule.counters.as<uint32_t>();

@@ -126,6 +126,17 @@ inline void uncharge(wc_budget* b, uint64_t bytes) {
   b->in_use.store(b->in_use.load() - bytes);
 }
 
+// Whether an allocation that is refused may have versions give back their
+// lane-major copies (give_back_lanes), and which one not to ask.
+struct Room {
+  bool make = true;
+  const wc_version* keep = nullptr;
+};
+// One of the versions that hold lane-major copies charged to `b` (or, with
+// `any`, on the current device) gives them back, unless it is in a call of
+// another thread's, `keep`, or a caller's graph walks them.  False: none did.
+bool give_back_lanes(wc_budget* b, bool any, const wc_version* keep);
+
 // A device buffer charged to a budget for its lifetime.
 struct DevBuf {
   void* ptr = nullptr;
@@ -158,10 +169,20 @@ struct DevBuf {
     bytes = 0;
   }
 
-  wc_status alloc(wc_budget* b, uint64_t n, wc_error_detail* d) {
+  wc_status alloc(wc_budget* b, uint64_t n, wc_error_detail* d, Room room = {}) {
     release();
     if (n == 0) n = 16;
     n = (n + 255) & ~uint64_t(255);
+    const wc_error_detail before = d ? *d : wc_error_detail{};
+    for (;;) {
+      const wc_status st = take(b, n, d);
+      if (st == WC_OK && d) *d = before;
+      if (st == WC_OK || !room.make || !give_back_lanes(b, st == WC_OUT_OF_MEMORY, room.keep))
+        return st;
+    }
+  }
+
+  wc_status take(wc_budget* b, uint64_t n, wc_error_detail* d) {
     WC_TRY(charge(b, n, d));
     cudaError_t e = cudaMalloc(&ptr, n);
     if (e != cudaSuccess) {
@@ -300,6 +321,14 @@ struct Locality {
   DevCsr csc;
 };
 
+// A version listed (while it lives) among those that may give back their
+// lane-major copies when memory is refused (version.cu).
+struct Lender {
+  wc_version* v = nullptr;
+  void list(wc_version* version);
+  ~Lender();
+};
+
 }  // namespace wc
 
 // The handle: one version's device copy, keyed by (graph, version).
@@ -316,6 +345,9 @@ struct wc_version {
   cudaStream_t stream = nullptr;
   wc::DevCsr fwd, rev;
   wc::Locality loc;                    // rev renumbered for the pull solvers
+  // A caller captured a walk of the lane-major copies into a graph of its own,
+  // which it may launch for as long as the version lives.
+  bool lanes_captured = false;
   bool reverse_given = false;          // the caller uploaded a reverse CSR
   std::vector<uint64_t> host_offsets;  // forward offsets, for truncated-BFS stats
   std::vector<uint64_t> host_rev_offsets;
@@ -345,6 +377,7 @@ struct wc_version {
   // Cursors open over the version (wc_bfs_cursor): it is not released
   // while any is.
   std::atomic<uint32_t> cursors{0};
+  wc::Lender lender;  // last: unlisted before any of the version goes
 };
 
 namespace wc {
@@ -393,6 +426,7 @@ struct Ctx {
   uint32_t timeout_ms;
 
   bool timing = false;
+  bool keep_lanes = false;  // this call's scratch has the version keep its lane-major copies
   bool capturing = false;  // the stream is being captured by run_captured
   bool device_error = false;  // finish() returned a status a kernel raised
   struct Timer {
@@ -551,7 +585,7 @@ struct Ctx {
     DevBuf& b = v->pool[tag];
     if (b.bytes < bytes) {
       b.release();
-      WC_TRY(b.alloc(budget, bytes + bytes / 8, detail));
+      WC_TRY(b.alloc(budget, bytes + bytes / 8, detail, Room{true, keep_lanes ? v : nullptr}));
     }
     *out = &b;
     return WC_OK;

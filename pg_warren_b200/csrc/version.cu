@@ -4,6 +4,7 @@
 #include <algorithm>
 #include <cstdlib>
 #include <memory>
+#include <set>
 #include <thread>
 
 #include "pagerank.h"
@@ -106,7 +107,8 @@ static wc_status put_rounds(wc_version* v, DevCsr& d, const std::vector<Unit>& u
   for (size_t q = 1; q < first.size(); q++) first[q] += first[q - 1];
   std::vector<Unit> ordered(units.size());
   for (const Unit& u : units) ordered[first[round_of(u)]++] = u;
-  WC_TRY(s.rounds.alloc(v->budget, std::max<size_t>(units.size(), 1) * sizeof(Unit), detail));
+  WC_TRY(s.rounds.alloc(v->budget, std::max<size_t>(units.size(), 1) * sizeof(Unit), detail,
+                        Room{false}));
   if (!units.empty())
     WC_CUDA(cudaMemcpy(s.rounds.ptr, ordered.data(), ordered.size() * sizeof(Unit),
                        cudaMemcpyHostToDevice), detail);
@@ -190,7 +192,58 @@ static wc_status put_fast_copies(wc_version* v, const std::vector<Unit>& rev_uni
     return device_lanes(v, v->fwd, v->host_offsets, v->rev, room, detail);
   }, &built));
   if (!built) v->fwd.lanes = LaneCsr{};
+  v->lender.list(v);
   return WC_OK;
+}
+
+static std::mutex g_lenders_mu;
+static std::set<wc_version*> g_lenders;
+
+void Lender::list(wc_version* version) {
+  std::lock_guard<std::mutex> lock(g_lenders_mu);
+  v = version;
+  g_lenders.insert(v);
+}
+Lender::~Lender() {
+  // Listed or not: whoever is taking its copies holds the list until done.
+  std::lock_guard<std::mutex> lock(g_lenders_mu);
+  g_lenders.erase(v);
+}
+
+// A version that gave its copies back does without from then on.  A call
+// takes the version's lock for as long as it reads them on the host, and no
+// call allocates between preparing a walk and queueing it; walks that are
+// queued are waited for.
+bool give_back_lanes(wc_budget* b, bool any, const wc_version* keep) {
+  std::lock_guard<std::mutex> list(g_lenders_mu);
+  int device = 0;
+  if (cudaGetDevice(&device) != cudaSuccess) return false;
+  for (auto it = g_lenders.begin(); it != g_lenders.end();) {
+    wc_version* v = *it;
+    if (v == keep || v->device != device || (!any && v->budget != b)) {
+      ++it;
+      continue;
+    }
+    std::unique_lock<std::recursive_mutex> lock(v->mu, std::try_to_lock);
+    if (!lock.owns_lock() || v->lanes_captured) {
+      ++it;
+      continue;
+    }
+    const bool holds = v->fwd.lanes.targets.ptr || v->rev.lanes.targets.ptr;
+    if (holds) {
+      if (cudaDeviceSynchronize() != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+      }
+      v->fwd.lanes = LaneCsr{};
+      v->rev.lanes = LaneCsr{};
+      v->loc.lane_targets.release();
+      v->loc.lane_hot.release();
+    }
+    it = g_lenders.erase(it);
+    if (holds) return true;
+  }
+  return false;
 }
 
 wc_status wc_device_check(wc_error_detail* detail) {
