@@ -47,8 +47,7 @@ __global__ void loc_degrees_kernel(const uint32_t* order, const uint32_t* roff, 
 // A warp per new row: the old row's entries in order, sources renumbered.
 __global__ void loc_entries_kernel(const uint32_t* order, const uint32_t* perm,
                                    const uint32_t* roff, const uint32_t* rtgt, const double* rw,
-                                   const int32_t* rwi, const uint32_t* noff, uint32_t n,
-                                   uint32_t* ntgt, double* nw, int32_t* nwi) {
+                                   const uint32_t* noff, uint32_t n, uint32_t* ntgt, double* nw) {
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
   for (uint32_t k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < n; k += warps) {
@@ -56,7 +55,6 @@ __global__ void loc_entries_kernel(const uint32_t* order, const uint32_t* perm,
     for (uint32_t e = a + lane; e < b; e += 32) {
       ntgt[dst + (e - a)] = perm[rtgt[e]];
       if (rw) nw[dst + (e - a)] = rw[e];
-      if (rwi) nwi[dst + (e - a)] = rwi[e];
     }
   }
 }
@@ -90,7 +88,6 @@ wc_status device_locality(wc_version* v, wc_error_detail* detail) {
   WC_TRY(c.offsets.alloc(v->budget, (n + 1) * 4 + kBulkPad, detail));
   WC_TRY(c.targets.alloc(v->budget, m * 4 + kBulkPad, detail));
   if (v->weighted) WC_TRY(c.weights.alloc(v->budget, m * 8 + kBulkPad, detail));
-  if (v->weighted && v->integral) WC_TRY(c.iweights.alloc(v->budget, m * 4 + kBulkPad, detail));
   if (n) {
     // Order: a stable radix sort of (¬length, id).
     DevBuf k0, k1, i1, temp;
@@ -129,8 +126,8 @@ wc_status device_locality(wc_version* v, wc_error_detail* detail) {
       note_launch(), loc_entries_kernel<<<max_blocks(8), 256, 0, st>>>(
           L.order.as<uint32_t>(), L.perm.as<uint32_t>(), v->rev.offsets.as<uint32_t>(),
           v->rev.targets.as<uint32_t>(), v->weighted ? v->rev.weights.as<double>() : nullptr,
-          c.iweights.ptr ? v->rev.iweights.as<int32_t>() : nullptr, c.offsets.as<uint32_t>(),
-          (uint32_t)n, c.targets.as<uint32_t>(), c.weights.as<double>(), c.iweights.as<int32_t>());
+          c.offsets.as<uint32_t>(), (uint32_t)n, c.targets.as<uint32_t>(),
+          c.weights.as<double>());
     WC_CUDA(cudaStreamSynchronize(st), detail);  // before the transient buffers go
   } else {
     WC_CUDA(cudaMemsetAsync(c.offsets.ptr, 0, 4, st), detail);

@@ -96,3 +96,17 @@ def test_an_upload_is_accepted_without_room_for_the_fast_copies(nodes, edges, we
             assert np.array_equal(got["pagerank"][1], got["noalloc"][1])
     if m > 32 * nodes:  # the copies are larger than any of the calls' scratch
         assert served == set(want)  # each of them without some copy
+
+
+def test_the_renumbered_copy_holds_no_integer_weights():
+    # Its readers (the ranks) take 64-bit weights.  What 64-bit weights add: 8
+    # bytes an entry of three row-major copies and a place of the two
+    # lane-major ones; what integer ones add to that: 4 an entry of two and a
+    # place of two.
+    g = W.gnm(2000, 40000, seed=6)
+    bytes_of = {k: version(g, w)[1].info().device_bytes for k, w in {
+        "none": None, "float": W.edge_weights(g, "uniform"), "int": W.edge_weights(g, "int")}.items()}
+    places = (bytes_of["float"] - bytes_of["none"] - 24 * g.edges) // 8
+    assert places >= 2 * g.edges
+    rounding = 4 * 256  # buffers come in multiples of 256 bytes
+    assert bytes_of["int"] - bytes_of["float"] <= 8 * g.edges + 4 * places + rounding
