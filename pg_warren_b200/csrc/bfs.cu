@@ -21,6 +21,7 @@
 
 #include "bfs.h"
 #include "operand.h"
+#include "row_chunks.h"
 #include "semiring.cuh"
 
 namespace wc {
@@ -261,10 +262,10 @@ __device__ inline uint32_t first_in_frontier(const uint32_t* tgt, const uint32_t
   uint32_t v[kPullEntries];
   uint32_t pos = hi;
 #pragma unroll
-  for (int q = 0; q < kPullEntries; q++) v[q] = lo + q < hi ? __ldg(tgt + lo + q) : 0u;
+  for (int q = 0; q < kPullEntries; q++) v[q] = in_row(lo, hi, q) ? __ldg(tgt + lo + q) : 0u;
 #pragma unroll
   for (int q = kPullEntries - 1; q >= 0; q--)
-    if (lo + q < hi && bit_at(fbits, v[q])) {
+    if (in_row(lo, hi, q) && bit_at(fbits, v[q])) {
       pos = lo + q;
       node = v[q];
     }
@@ -273,21 +274,20 @@ __device__ inline uint32_t first_in_frontier(const uint32_t* tgt, const uint32_t
     const int src = __ffs(rest) - 1;
     rest &= rest - 1;
     const uint32_t end = __shfl_sync(0xffffffffu, hi, src);
-    uint32_t e0 = __shfl_sync(0xffffffffu, lo, src) + kPullEntries;
-    for (; e0 < end; e0 += 32) {
-      const uint32_t e = e0 + lane;
+    const uint32_t from = __shfl_sync(0xffffffffu, lo, src) + kPullEntries;
+    each_chunk(from, end, 32, [&](uint64_t e0) {
+      const uint64_t e = e0 + lane;
       const uint32_t t = e < end ? __ldg(tgt + e) : 0u;
       const uint32_t hit = __ballot_sync(0xffffffffu, e < end && bit_at(fbits, t));
-      if (hit) {
-        const int first = __ffs(hit) - 1;
-        const uint32_t at = __shfl_sync(0xffffffffu, t, first);
-        if ((int)lane == src) {
-          pos = e0 + first;
-          node = at;
-        }
-        break;
+      if (!hit) return false;
+      const int first = __ffs(hit) - 1;
+      const uint32_t at = __shfl_sync(0xffffffffu, t, first);
+      if ((int)lane == src) {
+        pos = (uint32_t)e0 + first;
+        node = at;
       }
-    }
+      return true;
+    });
   }
   return pos;
 }
