@@ -217,6 +217,14 @@ __device__ inline void push_row_part(const LevelArgs& a, uint32_t u, uint32_t fi
   }
 }
 
+// Its blocks an SM: those that 40 registers a thread let be resident.  It runs
+// every level, long rows or none, and with eight an SM, a second wave of
+// blocks that only arrive, a search over a G(n, m) of 24,526 nodes with rows of
+// 11 took 118 µs in place of 108, over R-MAT 16 154 in place of 144 (over an
+// R-MAT of 262,144 nodes inwards 204 in place of 219: there the teams of a
+// block a row fill the second wave).
+constexpr int kPushBigBlocks = 6;
+
 __global__ void __launch_bounds__(256) push_big_kernel(LevelArgs a, SwitchArgs sw,
                                                        uint32_t next_is_last,
                                                        const int32_t* cancel) {
@@ -618,7 +626,7 @@ wc_status Search::advance(Ctx& ctx, uint32_t max_levels, bool defer_last) {
                     fb[(L + 2) % 3], (uint32_t)fw, big->as<uint32_t>(), big_cap, L + 1, (uint32_t)n,
                     depth_p, via_p, filter_dev};
         note_launch(), level_kernel<<<level_grid, 256, 0, ctx.stream>>>(a);
-        note_launch(), push_big_kernel<<<blocks, 256, 0, ctx.stream>>>(
+        note_launch(), push_big_kernel<<<max_blocks(kPushBigBlocks), 256, 0, ctx.stream>>>(
             a, sw, L + 1 >= max_depth ? 1u : 0u, v->cancel_dev);
       }
       WC_CUDA(cudaMemcpyAsync(plan, st, (kChunkLevels + 1) * sizeof(LevelState),
