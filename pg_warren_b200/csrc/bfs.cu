@@ -59,6 +59,7 @@ struct LevelArgs {
   uint32_t fwords;
   uint32_t* big;          // frontier rows too long for one warp
   uint32_t big_cap;       // its entries: long rows from the front, huge ones from the back
+  uint32_t big_rows;      // of which for long rows, the others for as many huge ones as can be
   uint32_t depth_next;
   uint32_t n;
   uint32_t* depth;
@@ -77,10 +78,16 @@ constexpr uint32_t kChunkLevels = 16;
 constexpr uint32_t kBigRow = 512;
 constexpr uint32_t kHugeRow = 32768;
 
-// The long-row list's entries: at most one per kBigRow entries of the rows
-// read (both CSRs for Both).
+// The long-row list's entries: one for every kListedRow entries of the rows
+// searched, and room for every huge row.  Long rows past it (a frontier of
+// many that are little over kBigRow) stay with their warps.
+constexpr uint32_t kListedRow = 2048;
+inline uint64_t searched_entries(uint64_t m, int dir) { return dir == WC_BOTH ? 2 * m : m; }
 inline uint32_t big_entries(uint64_t m, int dir) {
-  return (uint32_t)((m / kBigRow + 2) * (dir == WC_BOTH ? 2 : 1));
+  return (uint32_t)((m / kListedRow + 2) * (dir == WC_BOTH ? 2 : 1));
+}
+inline uint32_t big_list_rows(uint64_t m, int dir) {
+  return big_entries(m, dir) - (uint32_t)(searched_entries(m, dir) / kHugeRow);
 }
 
 // Appends the nodes v[q] that are taken (up to N a lane) to the next frontier
@@ -154,7 +161,7 @@ __device__ inline void offer_entries(const LevelArgs& a, const uint32_t* tgt, ui
 }
 
 // Push: a warp per frontier node, lanes over its row entries; rows longer
-// than kBigRow are listed for push_big_kernel instead.
+// than kBigRow are listed for push_big_kernel instead, where the list has room.
 __device__ inline void push_level(const LevelArgs& a) {
   const LevelState& st = *a.st;
   const unsigned lane = threadIdx.x & 31;
@@ -163,11 +170,15 @@ __device__ inline void push_level(const LevelArgs& a) {
     const uint32_t u = a.frontier[f];
     const uint32_t deg = a.adj.degree(u);
     if (deg > kBigRow) {
+      const bool huge = deg > kHugeRow;
+      uint32_t at = 0;
       if (lane == 0) {
-        if (deg > kHugeRow) a.big[a.big_cap - 1 - atomicAdd(&a.st->huge_count, 1u)] = u;
-        else a.big[atomicAdd(&a.st->big_count, 1u)] = u;
+        at = atomicAdd(huge ? &a.st->huge_count : &a.st->big_count, 1u);
+        if (huge) a.big[a.big_cap - 1 - at] = u;
+        else if (at < a.big_rows) a.big[at] = u;
       }
-      continue;
+      at = __shfl_sync(0xffffffffu, at, 0);
+      if (huge || at < a.big_rows) continue;
     }
     for (int part = 0; part < 2; part++) {
       const uint32_t* off = part == 0 ? a.adj.off0 : a.adj.off1;
@@ -236,7 +247,7 @@ __global__ void __launch_bounds__(256) push_big_kernel(LevelArgs a, SwitchArgs s
   for (uint32_t h = 0; h < huge; h++) push_row_part(a, a.big[a.big_cap - 1 - h], warp, warps);
   // Each long row gets a team of blocks: one when there are more rows than
   // blocks, else as many as share the grid evenly.
-  const uint32_t big = st.pull ? 0u : st.big_count;
+  const uint32_t big = st.pull ? 0u : min(st.big_count, a.big_rows);
   if (big) {
     const uint32_t team = max(1u, gridDim.x / big);
     const uint32_t rows_at_once = gridDim.x / team;
@@ -623,8 +634,8 @@ wc_status Search::advance(Ctx& ctx, uint32_t max_levels, bool defer_last) {
         const uint32_t L = d0 + q;
         LevelArgs a{adj, radj, st + q, queue[L & 1]->as<uint32_t>(),
                     queue[(L + 1) & 1]->as<uint32_t>(), fb[L % 3], fb[(L + 1) % 3],
-                    fb[(L + 2) % 3], (uint32_t)fw, big->as<uint32_t>(), big_cap, L + 1, (uint32_t)n,
-                    depth_p, via_p, filter_dev};
+                    fb[(L + 2) % 3], (uint32_t)fw, big->as<uint32_t>(), big_cap,
+                    big_list_rows(v->m, dir), L + 1, (uint32_t)n, depth_p, via_p, filter_dev};
         note_launch(), level_kernel<<<level_grid, 256, 0, ctx.stream>>>(a);
         note_launch(), push_big_kernel<<<max_blocks(kPushBigBlocks), 256, 0, ctx.stream>>>(
             a, sw, L + 1 >= max_depth ? 1u : 0u, v->cancel_dev);
