@@ -377,10 +377,19 @@ wc_status wc_version_upload(uint64_t graph_id, uint64_t version, const wc_csr_ho
   v->weighted = csr->weights != nullptr;
   WC_CUDA(cudaGetDevice(&v->device), detail);
   WC_CUDA(cudaStreamCreateWithFlags(&v->stream, cudaStreamNonBlocking), detail);
-  WC_TRY(put_csr(v.get(), v->fwd, csr->offsets, csr->targets, csr->weights, detail));
-  if (const wc_status outside = device_targets_in_space(v.get(), detail)) {
+  wc_status put = put_csr(v.get(), v->fwd, csr->offsets, csr->targets, csr->weights, detail);
+  if (put == WC_OK) put = device_targets_in_space(v.get(), detail);
+  // Arrays that are not a graph are that first, also where they do not fit.
+  if (put == WC_MEMORY_LIMIT || put == WC_OUT_OF_MEMORY)
+    for (uint64_t e = 0; e < m; e++)
+      if (csr->targets[e] >= n) {
+        if (detail) detail->node = csr->targets[e];
+        put = WC_NODE_OUTSIDE_ID_SPACE;
+        break;
+      }
+  if (put != WC_OK) {
     cudaStreamDestroy(v->stream);
-    return outside;
+    return put;
   }
   v->host_offsets.assign(csr->offsets, csr->offsets + n + 1);
   // The reverse CSR: the caller's, or a transpose on the device.
