@@ -110,12 +110,15 @@ static wc_status put_rounds(wc_version* v, DevCsr& d, const std::vector<Unit>& u
   WC_TRY(s.rounds.alloc(v->budget, std::max<size_t>(units.size(), 1) * sizeof(Unit), detail,
                         Room{false}));
   if (!units.empty())
-    WC_CUDA(cudaMemcpy(s.rounds.ptr, ordered.data(), ordered.size() * sizeof(Unit),
-                       cudaMemcpyHostToDevice), detail);
-  return WC_OK;
+    WC_CUDA(cudaMemcpyAsync(s.rounds.ptr, ordered.data(), ordered.size() * sizeof(Unit),
+                            cudaMemcpyHostToDevice, v->stream), detail);
+  return cuda_status(cudaStreamSynchronize(v->stream), detail, "batched units");
 }
 
-// The schedule of one orientation from its host offsets.
+// The schedule of one orientation from its host offsets.  Its copies are on the
+// version's stream, as the kernels are that read them: that stream does not
+// wait for the default one, and a copy from pageable memory there may still be
+// on its way to the device when cudaMemcpy returns.
 wc_status put_schedule(wc_version* v, DevCsr& d, const std::vector<uint64_t>& off,
                        wc_error_detail* detail, std::vector<Unit>* units_out) {
   std::vector<Unit> units;
@@ -124,10 +127,11 @@ wc_status put_schedule(wc_version* v, DevCsr& d, const std::vector<uint64_t>& of
   s.count = (uint32_t)units.size();
   WC_TRY(s.units.alloc(v->budget, std::max<size_t>(units.size(), 1) * sizeof(Unit), detail));
   if (!units.empty())
-    WC_CUDA(cudaMemcpy(s.units.ptr, units.data(), units.size() * sizeof(Unit),
-                       cudaMemcpyHostToDevice), detail);
+    WC_CUDA(cudaMemcpyAsync(s.units.ptr, units.data(), units.size() * sizeof(Unit),
+                            cudaMemcpyHostToDevice, v->stream), detail);
   WC_TRY(s.counters.alloc(v->budget, (uint64_t)std::max<uint32_t>(s.slots, 1) * 4, detail));
-  WC_CUDA(cudaMemset(s.counters.ptr, 0, (uint64_t)std::max<uint32_t>(s.slots, 1) * 4), detail);
+  WC_CUDA(cudaMemsetAsync(s.counters.ptr, 0, (uint64_t)std::max<uint32_t>(s.slots, 1) * 4,
+                          v->stream), detail);
   WC_TRY(s.carry.alloc(v->budget, (uint64_t)std::max<uint32_t>(s.slots, 1) * kCarryBytesPerSlot,
                        detail));
   // The long rows, for kernels that combine their pieces in a pass of their
@@ -143,10 +147,11 @@ wc_status put_schedule(wc_version* v, DevCsr& d, const std::vector<uint64_t>& of
   }
   WC_TRY(s.long_list.alloc(v->budget, std::max<size_t>(longs.size(), 4) * 4, detail));
   if (!longs.empty())
-    WC_CUDA(cudaMemcpy(s.long_list.ptr, longs.data(), longs.size() * 4, cudaMemcpyHostToDevice),
-            detail);
+    WC_CUDA(cudaMemcpyAsync(s.long_list.ptr, longs.data(), longs.size() * 4,
+                            cudaMemcpyHostToDevice, v->stream), detail);
   if (&d == &v->rev)
     WC_TRY(s.round_masks.alloc(v->budget, std::max<size_t>(units.size(), 1) * 4, detail));
+  WC_CUDA(cudaStreamSynchronize(v->stream), detail);
   if (units_out) *units_out = std::move(units);
   return WC_OK;
 }
@@ -193,7 +198,7 @@ static wc_status put_fast_copies(wc_version* v, const std::vector<Unit>& rev_uni
   }, &built));
   if (!built) v->fwd.lanes = LaneCsr{};
   v->lender.list(v);
-  return WC_OK;
+  return cuda_status(cudaStreamSynchronize(v->stream), detail, "version upload");
 }
 
 static std::mutex g_lenders_mu;
@@ -272,7 +277,7 @@ wc_status finish_version(wc_version* v, wc_error_detail* detail) {
   WC_TRY(put_schedule(v, v->rev, v->host_rev_offsets, detail, &rev_units));
   WC_TRY(device_locality(v, detail));
   WC_TRY(v->error.alloc(v->budget, sizeof(DeviceError), detail));
-  WC_CUDA(cudaMemset(v->error.ptr, 0, sizeof(DeviceError)), detail);
+  WC_CUDA(cudaMemsetAsync(v->error.ptr, 0, sizeof(DeviceError), v->stream), detail);
   // Four mapped words: the cancel word, then the pacing words (iterations
   // completed, done) that iterative kernels report to the host.
   WC_CUDA(cudaHostAlloc((void**)&v->cancel_host, 4 * sizeof(int32_t), cudaHostAllocMapped), detail);
