@@ -205,7 +205,8 @@ wc_status device_lanes(wc_version* v, DevCsr& d, const std::vector<uint64_t>& of
   }
   const uint32_t slices = cls.slice[2];
   const uint32_t first = slot * (kPieceEntries / 32);  // the slices' entries follow
-  L.count = (uint32_t)groups.size() + slices;
+  L.groups = (uint32_t)groups.size();
+  L.count = L.groups + slices;
   // A slice ends at its longest row, at most the shortest of the slice
   // before, so a class wastes at most one slice's entries, and less than a
   // step a slice where a row's lanes do not come out even.

@@ -374,15 +374,15 @@ __global__ void __launch_bounds__(kLaneThreads, 1)
 // most often as well.
 constexpr uint32_t kHotRows = 8192;
 
-// One iteration over the row-split schedule of the CSC in row order (lanes_pay
-// says when), or over a range of it (a part of a row-partitioned solve, which
-// gives no `longs`: its sums take a row in pieces as it comes).  Unweighted, four blocks an SM
-// (64 registers) keep more gathers in flight; with weights the extra
-// registers would spill, so three.  Bound by the latency of the gathers; with
-// plain loads in place of load_x_split's the parts of a weighted R-MAT 22 took
-// 1.05 ms whole and 0.30, 0.32 and 0.37 (first, second and last quarter), with
-// the split 0.97 and 0.29, 0.30 and 0.34 (an unweighted one 0.70 and 0.71
-// whole).
+// One iteration over the row-split schedule of the CSC in row order
+// (solve_lanes_pay says when), or over a range of it (a part of a
+// row-partitioned solve, which gives no `longs`: its sums take a row in pieces
+// as it comes).  Unweighted, four blocks an SM (64 registers) keep more gathers
+// in flight; with weights the extra registers would spill, so three.  Bound by
+// the latency of the gathers; with plain loads in place of load_x_split's the
+// parts of a weighted R-MAT 22 took 1.05 ms whole and 0.30, 0.32 and 0.37
+// (first, second and last quarter), with the split 0.97 and 0.29, 0.30 and
+// 0.34 (an unweighted one 0.70 and 0.71 whole).
 template <class W>
 __global__ void __launch_bounds__(kPullThreads, WSize<W>::v == 0 ? 4 : 3)
     pr_iter_kernel(CsrView<W> A, PrState s, uint32_t it, const uint4* longs, uint32_t long_count) {
@@ -596,7 +596,7 @@ wc_status PageRankRun::out_now(Ctx& ctx) {
 // 1,818,513 512 and 397, 131,072 and 1,942,324 541 and 474 (weighted 611 and
 // 615), but 262,144 and 2,016,841 554 and 568, 524,288 and 2,057,684 620 and
 // 663.  G(n, m) graphs have no long row: 65,536 and 262,129 260 and 290.
-static bool lanes_pay(const wc_version* v, bool weighted) {
+static bool solve_lanes_pay(const wc_version* v, bool weighted) {
   if (!v->rev.schedule.long_rows) return true;
   return v->m >= (!weighted && v->m >= 12 * v->n ? 1u << 21 : 1u << 20);
 }
@@ -606,10 +606,10 @@ wc_status PageRankRun::run(Ctx& ctx) {
   WC_TRY(launch_pr_init(s, grid, ctx.stream));
   PullLaunch L;
   WC_TRY(prepare_pull(ctx, v->rev, WC_PLUS_TIMES, opts.weighted, WC_F64, 1, L));
-  const bool lanes =
-      L.lanes && v->loc.lane_targets.ptr && lanes_pay(v, L.weight_kind == WEIGHTS_F64);
-  if (!lanes)
-    WC_TRY(prepare_pull(ctx, v->loc.csc, WC_PLUS_TIMES, opts.weighted, WC_F64, 1, L));
+  const bool lanes = v->rev.lanes.targets.ptr && v->loc.lane_targets.ptr &&
+                     solve_lanes_pay(v, L.weight_kind == WEIGHTS_F64);
+  if (lanes) L.lanes = &v->rev.lanes;
+  else WC_TRY(prepare_pull(ctx, v->loc.csc, WC_PLUS_TIMES, opts.weighted, WC_F64, 1, L));
   // No more blocks than the step keeps sums for.
   const uint32_t blocks = lanes ? std::min(lane_grid(L), grid) : grid;
   // With a tolerance the solve usually stops well before max_iter: the

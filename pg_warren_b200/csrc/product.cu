@@ -5,6 +5,7 @@
 #include <algorithm>
 #include <vector>
 
+#include "lanes.h"
 #include "operand.h"
 #include "product.h"
 #include "semiring.cuh"
@@ -30,6 +31,38 @@ size_t dtype_size(int dtype) {
   }
 }
 
+// Whether a product walks the lane-major copy (its results are the same either
+// way).  Over few entries its one block of 24 warps an SM is late to start and
+// each of its warps has one long slice or two, where the row-split schedule's
+// units are all alike; over many the schedule moves every product between
+// lanes.  Device time, schedule and lanes, µs.  G(n, m), f64 plus_times with
+// weights: 250,000 entries 8.3 and 10.3, 550,000 12.3 and 10.3, 900,000 15.1 and
+// 12.3; without, i64 min_plus, f32 or bool: 550,000 8.4, 10.0, 10.2, 8.2 and 10.3,
+// 11.7, 10.8, 10.3, 1,200,000 12.7, 14.4, 14.4, 12.3 and 12.4, 13.7, 12.4, 12.3;
+// in rows of 32, about the length from which a row has eight lanes, 1,600,000
+// 15.1, 16.5, 18.0, 12.3 and 16.5, 18.5, 16.5, 14.4.
+// R-MAT (long rows), f64 with weights: 679,000 19.3 and 22.6, 876,000 21.2 and
+// 22.6, 994,000 22.6 and 17.3, 1,240,000 22.9 and 18.5, in rows of 8 904,000
+// 20.5 and 23.8; the others, in rows of 16 and more: without weights 1,629,000
+// 22.6 and 23.3, 2,612,000 28.7 and 30.7, 3,692,000 41.0 and 32.9, i64 1,286,000
+// 20.6 and 22.0, 3,129,000 37.5 and 34.9; in rows of 8: 904,000 16.4 and 22.6,
+// 1,687,000 23.3 and 22.6 (i64 19.5 and 22.7, 26.7 and 24.8).
+// And where the long rows' units all but go round the warps, the longest slices
+// are every warp's second: 3,481 of them (1,819,000 entries, for 3,552 warps) f64
+// 30.8 and 38.9, without weights 24.5 and 36.9, 3,316 31.2 and 36.4, 24.6 and
+// 33.3; 2,891 29.7 and 26.6, 22.6 and 24.7.
+static bool lanes_pay(const wc_version* v, const DevCsr& csr, int weight_kind, int dtype) {
+  const uint64_t n = v->n, m = v->m;
+  const uint32_t groups = csr.lanes.groups;
+  const bool wide = weight_kind == WEIGHTS_F64 && dtype == WC_F64;
+  if (!csr.schedule.long_rows)
+    return m >= (wide ? 3u << 17 : m < 24 * n ? 3u << 18 : 5u << 19);
+  if (groups <= kLaneWarps && groups > kLaneWarps / 20 * 17) return false;
+  if (wide) return m >= (m < 8 * n ? 1u << 20 : 7u << 17);
+  if (m < 12 * n) return m >= 3u << 19;
+  return m >= (weight_kind == WEIGHTS_NONE ? 3u << 20 : 9u << 18);
+}
+
 // Fills a launch description for `csr` and the product.
 wc_status prepare_pull(Ctx& ctx, DevCsr& csr, int semiring, int weighted_flag, int dtype,
                        uint32_t width, PullLaunch& L) {
@@ -53,7 +86,8 @@ wc_status prepare_pull(Ctx& ctx, DevCsr& csr, int semiring, int weighted_flag, i
       L.lane_weights = csr.lanes.weights.ptr;
     }
   }
-  L.lanes = csr.lanes.count || csr.lanes.shorts ? &csr.lanes : nullptr;
+  const bool lanes = csr.lanes.count || csr.lanes.shorts;
+  L.lanes = lanes && lanes_pay(v, csr, L.weight_kind, dtype) ? &csr.lanes : nullptr;
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   if (L.lanes && ctx.stream && cudaStreamIsCapturing(ctx.stream, &cs) == cudaSuccess &&
       cs != cudaStreamCaptureStatusNone)
@@ -129,12 +163,6 @@ static wc_status product(wc_version* v, const wc_call* call, const wc_product* p
     L.unit_count = uc[part + 1] - uc[part];
     L.lanes = nullptr;  // a range of the rows: over the row-split schedule
   }
-  // Under a million entries in rows of fewer than eight, the row-split schedule
-  // too: the lane-major copy's one block of 24 warps an SM is late to start and
-  // a warp's slice is over in a few steps (f64 plus_times, lanes and schedule:
-  // G(n, m) of 5,000 nodes and 30,000 entries 42 and 36 µs, R-MAT of 160,000
-  // nodes and 960,000 entries 55 and 47; R-MAT 16 with rows of 16 45 and 56).
-  if (v->m < (1u << 20) && v->m < 8 * v->n) L.lanes = nullptr;
   if (width > 1) {
     DevBuf* mc;
     WC_TRY(ctx.scratch(POOL_SPMM_CARRY,

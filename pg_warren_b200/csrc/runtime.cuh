@@ -291,7 +291,7 @@ struct LaneCsr {
   DevBuf rows, lengths;      // u32 / u16: row ids sorted by length, longest first; their entries
   DevBuf targets, weights, iweights;
   DevBuf hot;                // u32[hot_count]: the hot nodes, most gathered first
-  uint32_t count = 0;
+  uint32_t count = 0, groups = 0;   // of the units, the first `groups` are long rows' pieces
   uint32_t filled = 0, shorts = 0;  // of `rows`: those with entries, then to here the empty ones
   uint32_t hot_count = 0;
   uint32_t run = 1;     // pieces of a long row a unit takes at most

@@ -27,7 +27,7 @@ def products(gv):
 
 
 def graph():
-    return W.gnm(3001, 240000, seed=2)
+    return W.gnm(300007, 3000000, seed=2)  # enough entries for its products to walk the copies
 
 
 def copies(g):

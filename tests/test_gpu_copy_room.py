@@ -60,7 +60,7 @@ def calls(g, gv, weights):
     return out
 
 
-@pytest.mark.parametrize("nodes,edges,weighted", [(3001, 240000, False), (3001, 240000, True),
+@pytest.mark.parametrize("nodes,edges,weighted", [(6007, 900000, False), (6007, 900000, True),
                                                   (40000, 300000, False), (9, 0, False)])
 def test_an_upload_is_accepted_without_room_for_the_fast_copies(nodes, edges, weighted):
     g = W.gnm(nodes, edges, seed=2)
