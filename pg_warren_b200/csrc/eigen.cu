@@ -576,6 +576,13 @@ struct Eigensolver {
 
   cudaStream_t st() const { return ctx.stream; }
 
+  // A copy on the call's stream, there when it returns.  (cudaMemcpy goes by
+  // the default stream, which the call's kernels neither wait for nor hold up.)
+  wc_status copy(void* dst, const void* src, uint64_t bytes) {
+    WC_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDefault, st()), ctx.detail);
+    return cuda_status(cudaStreamSynchronize(st()), ctx.detail, "copy");
+  }
+
   wc_status sum_final(uint32_t count, uint32_t columns, double* out_host) {
     if ((uint64_t)count * columns > kSumFinalMaxValues) return WC_INVALID_ARGUMENT;
     note_launch(), sum_final_kernel<<<1, 256, 0, st()>>>(
@@ -642,8 +649,8 @@ struct Eigensolver {
       WC_TRY(prepare_pull(ctx, v->rev, WC_PLUS_TIMES, o.weighted, WC_F64, 1, R));
       WC_TRY(launch_pull(R, WC_F64, input->ptr, scratch->ptr));
       std::vector<double> ax(n), atx(n);
-      WC_CUDA(cudaMemcpy(ax.data(), output->ptr, nb, cudaMemcpyDeviceToHost), ctx.detail);
-      WC_CUDA(cudaMemcpy(atx.data(), scratch->ptr, nb, cudaMemcpyDeviceToHost), ctx.detail);
+      WC_TRY(copy(ax.data(), output->ptr, nb));
+      WC_TRY(copy(atx.data(), scratch->ptr, nb));
       double size = 0.0, diff = 0.0;
       bool nan = false;
       for (uint32_t i = 0; i < n; i++) {
@@ -670,7 +677,7 @@ struct Eigensolver {
       return (wc_status)e.status;
     }
     std::vector<uint8_t> act(n);
-    WC_CUDA(cudaMemcpy(act.data(), active->ptr, n, cudaMemcpyDeviceToHost), ctx.detail);
+    WC_TRY(copy(act.data(), active->ptr, n));
     dimension = 0;
     for (uint8_t a : act) dimension += a;
     return WC_OK;
@@ -700,15 +707,15 @@ struct Eigensolver {
     // Number the roots (active, own parent) in node order.
     std::vector<uint32_t> ph(n);
     std::vector<uint8_t> act(n);
-    WC_CUDA(cudaMemcpy(ph.data(), par, (uint64_t)n * 4, cudaMemcpyDeviceToHost), ctx.detail);
-    WC_CUDA(cudaMemcpy(act.data(), active->ptr, n, cudaMemcpyDeviceToHost), ctx.detail);
+    WC_TRY(copy(ph.data(), par, (uint64_t)n * 4));
+    WC_TRY(copy(act.data(), active->ptr, n));
     std::vector<uint32_t> number(n, 0);
     components = 0;
     for (uint32_t i = 0; i < n; i++)
       if (act[i] && ph[i] == i) number[i] = (uint32_t)components++;
     std::vector<uint32_t> cm(n, 0);
     for (uint32_t i = 0; i < n; i++) cm[i] = act[i] ? number[ph[i]] : 0;
-    WC_CUDA(cudaMemcpy(comp->ptr, cm.data(), (uint64_t)n * 4, cudaMemcpyHostToDevice), ctx.detail);
+    WC_TRY(copy(comp->ptr, cm.data(), (uint64_t)n * 4));
     colour = bip = nullptr;
     bipartite_host.assign(components, 0);
     if (need_colours) {
@@ -721,12 +728,12 @@ struct Eigensolver {
       Search s;
       WC_TRY(s.run(ctx, WC_BOTH, roots.data(), roots.size(), WC_UNREACHED, nullptr, GPU_SWITCH));
       std::vector<uint32_t> depth(n);
-      WC_CUDA(cudaMemcpy(depth.data(), s.depth_p, (uint64_t)n * 4, cudaMemcpyDeviceToHost), ctx.detail);
+      WC_TRY(copy(depth.data(), s.depth_p, (uint64_t)n * 4));
       std::vector<uint8_t> col(n, 0);
       for (uint32_t i = 0; i < n; i++) col[i] = act[i] && depth[i] != WC_UNREACHED ? (depth[i] & 1) : 0;
       std::vector<uint64_t> off(v->host_offsets);
       std::vector<uint32_t> tgt(v->m);
-      WC_CUDA(cudaMemcpy(tgt.data(), v->fwd.targets.ptr, v->m * 4, cudaMemcpyDeviceToHost), ctx.detail);
+      WC_TRY(copy(tgt.data(), v->fwd.targets.ptr, v->m * 4));
       std::vector<uint8_t> odd(components, 0);
       for (uint32_t u = 0; u < n; u++) {
         if (!act[u]) continue;
@@ -738,9 +745,9 @@ struct Eigensolver {
       for (uint64_t c = 0; c < components; c++) bipartite_host[c] = !odd[c];
       WC_TRY(ctx.scratch(POOL_ADJ_2, n, &colour));
       WC_TRY(ctx.scratch(POOL_ADJ_3, std::max<uint64_t>(components, 1), &bip));
-      WC_CUDA(cudaMemcpy(colour->ptr, col.data(), n, cudaMemcpyHostToDevice), ctx.detail);
+      WC_TRY(copy(colour->ptr, col.data(), n));
       if (components)
-        WC_CUDA(cudaMemcpy(bip->ptr, bipartite_host.data(), components, cudaMemcpyHostToDevice), ctx.detail);
+        WC_TRY(copy(bip->ptr, bipartite_host.data(), components));
     }
     return WC_OK;
   }
@@ -768,7 +775,7 @@ struct Eigensolver {
       WC_TRY(prepare_pull(ctx, v->fwd, WC_MIN_FIRST, o.weighted, WC_F64, 1, L));
       WC_TRY(launch_pull(L, WC_F64, input->ptr, output->ptr));
       std::vector<double> mins(n);
-      WC_CUDA(cudaMemcpy(mins.data(), output->ptr, (uint64_t)n * 8, cudaMemcpyDeviceToHost), ctx.detail);
+      WC_TRY(copy(mins.data(), output->ptr, (uint64_t)n * 8));
       nonnegative = true;
       for (double m : mins)
         if (m != m || m < 0.0) nonnegative = false;
@@ -985,7 +992,7 @@ struct Eigensolver {
   wc_status combine(const RitzPairs& r, uint32_t l, double* out) {
     std::vector<double> vl(len);
     for (uint32_t i = 0; i < len; i++) vl[i] = r.vectors[(size_t)i * len + l];
-    WC_CUDA(cudaMemcpy(vbuf->ptr, vl.data(), len * 8, cudaMemcpyHostToDevice), ctx.detail);
+    WC_TRY(copy(vbuf->ptr, vl.data(), len * 8));
     note_launch(), rotate_kernel<<<grid, 256, 0, st()>>>(n, Q->as<double>(), vbuf->as<double>(), len, 1, 1, out);
     return cuda_status(cudaGetLastError(), ctx.detail, "combine");
   }
@@ -1007,7 +1014,7 @@ struct Eigensolver {
     }
     if (keep_vector) {
       p.vector.resize(n);
-      WC_CUDA(cudaMemcpy(p.vector.data(), x, (uint64_t)n * 8, cudaMemcpyDeviceToHost), ctx.detail);
+      WC_TRY(copy(p.vector.data(), x, (uint64_t)n * 8));
     }
     return WC_OK;
   }
@@ -1032,7 +1039,7 @@ struct Eigensolver {
       WC_CUDA(cudaMemcpyAsync(&at, idx, 4, cudaMemcpyDeviceToHost, st()), ctx.detail);
       WC_CUDA(cudaStreamSynchronize(st()), ctx.detail);
       double xv = 0.0;
-      WC_CUDA(cudaMemcpy(&xv, x + at, 8, cudaMemcpyDeviceToHost), ctx.detail);
+      WC_TRY(copy(&xv, x + at, 8));
       sign = xv < 0 ? -1.0 : 1.0;
     }
     note_launch(), scale_vec_kernel<<<grid, 256, 0, st()>>>(x, n, sign / norm);
@@ -1081,7 +1088,7 @@ struct Eigensolver {
       std::vector<double> vk((size_t)len * kept);
       for (uint32_t i = 0; i < len; i++)
         for (uint32_t l = 0; l < kept; l++) vk[(size_t)i * kept + l] = r.vectors[(size_t)i * len + l];
-      WC_CUDA(cudaMemcpy(vbuf->ptr, vk.data(), vk.size() * 8, cudaMemcpyHostToDevice), ctx.detail);
+      WC_TRY(copy(vbuf->ptr, vk.data(), vk.size() * 8));
       note_launch(), rotate_kernel<<<grid, 256, 0, st()>>>(n, Q->as<double>(), vbuf->as<double>(), len, kept, kept,
                                             Q2->as<double>());
       WC_CUDA(cudaMemcpyAsync(Q->ptr, Q2->ptr, (uint64_t)kept * n * 8, cudaMemcpyDeviceToDevice, st()),
@@ -1220,7 +1227,7 @@ wc_status wc_eigen(wc_version* v, const wc_call* call, const wc_eigen_opts* opts
     const Pair& p = all[ord[q]];
     values[q] = p.value;
     residuals[q] = p.residual;
-    if (keep) WC_CUDA(cudaMemcpy(vectors + q * v->n, p.vector.data(), v->n * 8, cudaMemcpyDefault), ctx.detail);
+    if (keep) WC_TRY(es.copy(vectors + q * v->n, p.vector.data(), v->n * 8));
     if (ord[q] < known_count) exact_count++;
   }
   if (stats) {
