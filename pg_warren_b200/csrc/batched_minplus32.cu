@@ -53,17 +53,17 @@ constexpr uint32_t kMp32Warps = 4;    // warps a block
 constexpr uint32_t kMp32Rows = 16;    // rows whose minima wait to be settled
 constexpr uint32_t kMp32Unroll = 16;  // entries gathered at once
 
-// A lane's columns of a row.
-template <int C> struct alignas(4 * C) Cols32 { int32_t v[C]; };
+// A lane's columns of a row of 64 (the row kernel).
+struct alignas(8) Cols32 { int32_t v[2]; };
 
-__device__ inline Cols32<2> load_cols(const Cols32<2>* p) {
+__device__ inline Cols32 load_cols(const Cols32* p) {
   const int2 v = __ldg(reinterpret_cast<const int2*>(p));
-  return Cols32<2>{{v.x, v.y}};
+  return Cols32{{v.x, v.y}};
 }
 
 // A warp's shared memory: the unit's hits and the rows' minima.
-template <int P> struct Mp32Warp {
-  Cols32<P / 32> y[kMp32Rows][32];
+struct Mp32Warp {
+  Cols32 y[kMp32Rows][32];
   uint32_t j[kTileEntries];
   int32_t w[kTileEntries];
 };
@@ -329,25 +329,24 @@ __global__ void __launch_bounds__(256, 3) mp32_tile_kernel(Mp32 s, uint32_t it) 
 // out of L2): sixteen rows in flight a warp, twenty warps an SM, where the
 // kernel that kept per-row minima in shared memory had two half-warps' eight
 // in flight in sixteen warps.
-template <int P>
 __global__ void __launch_bounds__(32 * kMp32Warps, 5) mp32_iter_kernel(Mp32 s, uint32_t it) {
-  constexpr int C = P / 32;
+  constexpr int P = 64, C = 2;
   constexpr int Q = kTileEntries / 32;
   constexpr uint32_t U = kMp32Unroll;
-  typedef Cols32<C> Cols;
+  typedef Cols32 Cols;
   uint32_t running[C], any_running = 0;
 #pragma unroll
   for (int c = 0; c < C; c++) any_running |= running[c] = s.running[c];
   if (!any_running) return;
-  __shared__ Mp32Warp<P> sm_all[kMp32Warps];
-  Mp32Warp<P>& sm = sm_all[threadIdx.x >> 5];
+  __shared__ Mp32Warp sm_all[kMp32Warps];
+  Mp32Warp& sm = sm_all[threadIdx.x >> 5];
   const unsigned lane = threadIdx.x & 31;
   // The lane's columns C·lane .. C·lane + C - 1: which of them still run.
   uint32_t run = 0;
 #pragma unroll
   for (int c = 0; c < C; c++) {
     const uint32_t col = C * lane + c;
-    run |= ((running[C == 1 ? 0 : col >> 5] >> (col & 31)) & 1u) << c;
+    run |= ((running[col >> 5] >> (col & 31)) & 1u) << c;
   }
   const uint32_t* fell_cur = s.fell_rows[it & 1];
   uint32_t* fell_next = s.fell_rows[(it + 1) & 1];
@@ -527,7 +526,8 @@ __global__ void __launch_bounds__(32 * kMp32Warps, 5) mp32_iter_kernel(Mp32 s, u
 // Rows of 32 columns stay in tiles, four columns a lane (32 searches over an
 // R-MAT of 120,000 nodes: 633 µs, 950 with one column a lane).
 inline bool mp32_rows(const Schedule& s) {
-  return 4ull * (s.count - s.tiles) >= s.count && s.count >= (uint32_t)max_blocks((int)kMp32Blocks) * kMp32Warps / 2;
+  return 4ull * (s.count - s.tiles) >= s.count &&
+         s.count >= (uint32_t)max_blocks((int)kMp32Blocks) * kMp32Warps / 2;
 }
 
 // Copies the rows that fell into the iterate; clears the bitmap the
@@ -643,7 +643,7 @@ wc_status mp32_pass(Ctx& ctx, const uint64_t* sources, const uint32_t* caps, con
       max_blocks(8), (uint32_t)((words + 7) / 8)));
   for (uint32_t it = 0; it < max_cap; it++) {
     if (rows) {
-      note_launch(), mp32_iter_kernel<64><<<grid, 32 * kMp32Warps, 0, st>>>(s, it);
+      note_launch(), mp32_iter_kernel<<<grid, 32 * kMp32Warps, 0, st>>>(s, it);
     } else {
       note_launch(), mp32_tile_kernel<P><<<grid, 256, smem, st>>>(s, it);
     }
