@@ -85,7 +85,7 @@ static wc_status static_setup(Ctx& ctx, PageRankRun& run, const wc_pagerank_opts
   if (o->has_tol && o->max_iter > 0)
     WC_TRY((wc_status)sql_float<F_MUL>(run.nodes, o->tol, &threshold));
   run.grid = pagerank_grid(v->loc.csc);
-  const uint32_t blocks = pagerank_partial_blocks(v->loc.csc);  // block sums kept
+  const uint32_t blocks = run.grid;  // block sums kept
 
   unsigned char* p = base;
   auto take = [&](uint64_t bytes) {
@@ -210,7 +210,7 @@ wc_status wc_pagerank_noalloc(wc_version* v, const wc_call* call, const wc_pager
     set_message(detail, "a personalised PageRank needs per-call memory; use wc_pagerank");
     return WC_UNSUPPORTED;
   }
-  const uint32_t blocks = pagerank_partial_blocks(v->loc.csc);
+  const uint32_t blocks = pagerank_grid(v->loc.csc);
   const uint64_t need = static_bytes(v->n, o->max_iter, blocks, tombstones != nullptr);
   if (need > kStaticScratchBytes) {
     if (detail) {

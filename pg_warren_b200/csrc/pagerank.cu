@@ -457,13 +457,6 @@ uint64_t live_count(const uint64_t* tomb, uint64_t n) {
   return n - dead;
 }
 
-// The sums of pagerank_grid blocks, and room that the working memory of
-// wc_pagerank_noalloc has always counted beside them.
-uint32_t pagerank_partial_blocks(const DevCsr& csc) {
-  return pagerank_grid(csc) +
-         std::max<uint32_t>(1, std::min<uint32_t>((csc.schedule.long_rows + 7) / 8, max_blocks(2)));
-}
-
 uint32_t pagerank_grid(const DevCsr& csc) {
   return std::max<uint32_t>(1, std::min<uint32_t>((csc.schedule.count + kPullWarps - 1) / kPullWarps,
                                                   max_blocks(8)));
@@ -493,11 +486,10 @@ wc_status PageRankRun::setup(Ctx& ctx, const wc_pagerank_opts* o, const uint64_t
   double threshold = 0.0;
   if (o->has_tol && o->max_iter > 0) WC_TRY((wc_status)sql_float<F_MUL>(nodes, o->tol, &threshold));
   grid = pagerank_grid(v->loc.csc);
-  const uint32_t partial_blocks = pagerank_partial_blocks(v->loc.csc);
   WC_TRY(ctx.scratch(POOL_PR_X, 2 * n * 8, &x));
   WC_TRY(ctx.scratch(POOL_PR_MSG, 2 * n * 8, &msg));
   WC_TRY(ctx.scratch(POOL_PR_OUT, n * 8, &out));
-  const uint64_t scalar_bytes = (2 * (uint64_t)o->max_iter + 8) * 8 + 2 * partial_blocks * 8 + 64;
+  const uint64_t scalar_bytes = (2 * (uint64_t)o->max_iter + 8) * 8 + 2 * (uint64_t)grid * 8 + 64;
   WC_TRY(ctx.scratch(POOL_PR_SCALARS, scalar_bytes, &scalars));
   uint64_t* tomb_dev = nullptr;
   if (th) {
@@ -527,7 +519,7 @@ wc_status PageRankRun::setup(Ctx& ctx, const wc_pagerank_opts* o, const uint64_t
   s.delta = sc;
   s.dangling = sc + o->max_iter;
   s.partials = sc + 2 * (uint64_t)o->max_iter + 8;
-  unsigned char* tail = reinterpret_cast<unsigned char*>(s.partials + 2 * partial_blocks);
+  unsigned char* tail = reinterpret_cast<unsigned char*>(s.partials + 2 * grid);
   s.counter = reinterpret_cast<unsigned*>(tail);
   s.iterations = reinterpret_cast<uint32_t*>(tail + 8);
   s.done = reinterpret_cast<int32_t*>(tail + 16);

@@ -64,8 +64,7 @@ void pagerank_part_forget(const wc_version* v);
 // The row-partitioned search's and product's state kept with a version
 // (bfs_part.cu), dropped when the version is released.
 void bfs_part_forget(const wc_version* v);
-// Blocks of an iteration launch over `csc`, and the block sums kept for it.
+// Blocks of an iteration launch over `csc` at the most, each with a block sum.
 uint32_t pagerank_grid(const DevCsr& csc);
-uint32_t pagerank_partial_blocks(const DevCsr& csc);
 
 }  // namespace wc
