@@ -97,6 +97,8 @@ wc_status prepare_pull(Ctx& ctx, DevCsr& csr, int semiring, int weighted_flag, i
   L.counters = csr.schedule.counters.as<uint32_t>();
   L.carry = csr.schedule.carry.ptr;
   L.n = (uint32_t)v->n;
+  L.entries = v->m;
+  L.skewed = csr.schedule.long_rows != 0;
   L.width = width;
   L.semiring = semiring;
   L.max_blocks = max_blocks(8);

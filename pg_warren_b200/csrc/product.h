@@ -34,6 +34,8 @@ struct PullLaunch {
   void* carry;
   void* carry_multi;  // width > 1: 32 partials a long-row slot
   uint32_t n;
+  uint64_t entries;
+  bool skewed;  // some rows are in pieces
   uint32_t width;
   int32_t semiring;
   uint32_t max_blocks;

@@ -7,14 +7,15 @@
 // where X allows it), and the warp's G = 32 / LPR lane groups each take a run
 // of the tile's rows of about equal entries.  A group gathers up to eight of a
 // row's entries at once and folds them in ascending order, the reference's
-// order (compute/product/kernel.rs:184-198) to the bit.  A long row's piece is split between the groups as contiguous
-// runs, combined left to right, and a row's pieces in piece order by the last
-// to finish.
+// order (compute/product/kernel.rs:184-198) to the bit.  A long row's piece is
+// split between the groups as contiguous runs, combined left to right, and a
+// row's pieces in piece order by the last to finish.
 //
 // What bounds it: the latency of the gathers of X's rows, row after row of a
-// group.  The kernel this replaces had a group's offsets, targets and gathers
-// one after another, a lane a column: 16 f32 columns over an R-MAT graph of
-// 300,007 nodes and 4.6 M entries took 405 µs, 196 now.
+// group.  pull_multi, which runs the blocks that this does not pay for
+// (spmm_rows_pay), has a group's offsets, targets and gathers one after another,
+// a lane a column: 16 weighted f32 columns over an R-MAT graph of 300,007 nodes
+// and 4.6 M entries take it 405 µs, 196 here.
 #pragma once
 
 #include "pull.cuh"
