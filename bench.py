@@ -458,6 +458,11 @@ def leg_c3(W, O, torch, dev, stream, peak, g=None):
     plain_s, plain_cols, plain_iters = 0.0, 0, 0
     xs = torch.empty(n, dtype=torch.int64, device=dev)
     ys = torch.empty(n, dtype=torch.int64, device=dev)
+    xs.fill_(np.iinfo(np.int64).max)
+    for _ in range(3):  # untimed: the loop's kernels and buffers are warm
+        ys.copy_(xs)
+        W.spmv(gv, prod, xs, ys)
+        (ys < xs).any().item()
     for q in range(8):
         xs.fill_(np.iinfo(np.int64).max)
         xs[int(src[q])] = 0

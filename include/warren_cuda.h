@@ -353,7 +353,7 @@ wc_status wc_pagerank_noalloc(wc_version* version, const wc_call* call,
 
 /* No reference counterpart (warren-core solves on one host): one rank's part
  * of a row-partitioned PageRank over several GPUs.  The solve's rows (the
- * numbering wc_pagerank iterates in: nodes by out-degree, largest first) are
+ * numbering wc_pagerank iterates in: nodes by in-degree, largest first) are
  * cut into `parts` ranges of about equal entries; every rank holds the whole
  * version and pulls its range each iteration, and between iterations the
  * caller sums the parts' L1 changes and dangling ranks and gathers the

@@ -785,8 +785,10 @@ __global__ void __launch_bounds__(kDepthBlock, 1)
     // as 127 (the one-subtraction compare of phase 2 needs caps <= 127).
     cap4s[x] = (x < k ? min(caps[x], NB == 5 ? 127u : 255u) : 0u) * 0x01010101u;
   }
-  // Word and 16-byte stores need the rows (and the caller's buffer) to
-  // start on such boundaries; otherwise bytes are stored one at a time.
+  // 16-byte stores need the rows (and the caller's buffer) to start on such
+  // boundaries.  Otherwise a whole tile's runs are shifted to the words that
+  // they cover, and the last tile is stored by word where the rows start on
+  // one, else by byte.
   const uintptr_t base = reinterpret_cast<uintptr_t>(depth_out);
   const bool aligned = (n & 3u) == 0 && (base & 3u) == 0;
   const bool aligned16 = (n & 15u) == 0 && (base & 15u) == 0;
