@@ -588,7 +588,7 @@ wc_status PageRankRun::out_now(Ctx& ctx) {
 // 1,818,513 512 and 397, 131,072 and 1,942,324 541 and 474 (weighted 611 and
 // 615), but 262,144 and 2,016,841 554 and 568, 524,288 and 2,057,684 620 and
 // 663.  G(n, m) graphs have no long row: 65,536 and 262,129 260 and 290.
-static bool solve_lanes_pay(const wc_version* v, bool weighted) {
+bool solve_lanes_pay(const wc_version* v, bool weighted) {
   if (!v->rev.schedule.long_rows) return true;
   return v->m >= (!weighted && v->m >= 12 * v->n ? 1u << 21 : 1u << 20);
 }

@@ -51,6 +51,8 @@ struct PageRankRun {
   wc_status result(Ctx& ctx, double* ranks, uint32_t* iterations, double* margin);
 };
 
+// Whether a solve walks the reverse lane-major copy, where it is there.
+bool solve_lanes_pay(const wc_version* v, bool weighted);
 uint64_t live_count(const uint64_t* tomb, uint64_t n);
 // pr_init_kernel: the start vector, its messages and dangling rank.
 wc_status launch_pr_init(const PrState& s, uint32_t grid, cudaStream_t stream);

@@ -63,6 +63,12 @@ static bool lanes_pay(const wc_version* v, const DevCsr& csr, int weight_kind, i
   return m >= (weight_kind == WEIGHTS_NONE ? 3u << 20 : 9u << 18);
 }
 
+bool any_product_walks_lanes(const wc_version* v, const DevCsr& csr) {
+  if (lanes_pay(v, csr, WEIGHTS_NONE, WC_F64)) return true;
+  if (!v->weighted) return false;
+  return lanes_pay(v, csr, WEIGHTS_F64, WC_F64) || lanes_pay(v, csr, WEIGHTS_F64, WC_F32);
+}
+
 // Fills a launch description for `csr` and the product.
 wc_status prepare_pull(Ctx& ctx, DevCsr& csr, int semiring, int weighted_flag, int dtype,
                        uint32_t width, PullLaunch& L) {

@@ -49,6 +49,10 @@ struct PullLaunch {
   const void* lane_weights;
 };
 
+// Whether any product over `csr` would walk a lane-major copy of it (its
+// schedule is there).
+bool any_product_walks_lanes(const wc_version* v, const DevCsr& csr);
+
 // Cuts `csr`'s schedule into `parts` ranges of about equal entries at unit
 // boundaries (a long row's pieces in one range): unit_cut and row_cut get
 // parts + 1 entries, the parts' first units and first rows.
