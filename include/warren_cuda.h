@@ -242,7 +242,10 @@ typedef struct wc_version_info {
 /* Uploads `csr` for (graph_id, version) to the current device: the derived
  * device copy the seam keys by version (the reference's design document,
  * line 1240).  Charged to
- * `budget` (the version holds it until wc_version_release). */
+ * `budget` (the version holds it until wc_version_release).  Copies that only
+ * make calls faster are left out where the budget or the device has no room
+ * for them, and given back (device_bytes falls) when another upload or a call's
+ * working memory is refused. */
 wc_status wc_version_upload(uint64_t graph_id, uint64_t version, const wc_csr_host* csr,
                             wc_budget* budget, const wc_call* call, wc_version** out);
 wc_status wc_version_release(wc_version* version);

@@ -18,9 +18,10 @@
 // The code is kept to one copy of each loop: a small graph's launch is over
 // in the time its instructions take to arrive.
 //
-// R-MAT 22 (65 M entries): the weighted f64 plus_times product 768 -> 382 µs,
-// a PageRank solve of 10 iterations 5.89 -> 3.84 ms; min_plus over i64 on a
-// G(n, m) of 16 M entries 117 -> 98 µs; PageRank on R-MAT 16 412 -> 335 µs.
+// R-MAT 22 (65 M entries): the weighted f64 plus_times product 768 -> 381 µs,
+// a PageRank solve of 10 iterations 5.89 -> 3.53 ms; min_plus over i64 on a
+// G(n, m) of 16 M entries 116 -> 98 µs.  Over few entries the row-split schedule
+// is the faster: lanes_pay (product.cu), solve_lanes_pay (pagerank.cu).
 #pragma once
 
 #include "lanes.h"

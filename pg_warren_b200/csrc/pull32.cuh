@@ -19,7 +19,7 @@
 // a row-end test where its sixteen are not inside one row: 16 warp
 // instructions with the rows' updates, against 32 for the pull that staged
 // every row in shared memory.  Personalised PageRank of 64 sets on R-MAT 20
-// 48.3 -> 40.9 ms; the adjoint of 32 losses on R-MAT 18 42.1 -> 29.4 ms.
+// 45.1 -> 36.0 ms; the adjoint of 32 losses on R-MAT 18 45.3 -> 28.8 ms.
 //
 // The solver's epilogue `Epi` provides:
 //   Row                      per-row values, loaded by the tile's lane r for
